@@ -287,6 +287,20 @@ struct Ops<c64, zdd> {
   }
 };
 
+// The entry of a Gram matrix mirrored across the diagonal: the same sum, for A^H A its conjugate
+template <typename T, typename Acc>
+__device__ __forceinline__ Acc gram_mirror(Acc s) {
+  return s;
+}
+template <>
+__device__ __forceinline__ c32h gram_mirror<c32h, c32h>(c32h s) {
+  return {s.x, -s.y};
+}
+template <>
+__device__ __forceinline__ c64h gram_mirror<c64h, c64h>(c64h s) {
+  return {s.x, -s.y};
+}
+
 // ---------------------------------------------------------------- device error word
 // Kernels never trap.  A wait that runs out of iterations records a code here and returns.
 enum : int { SKINNY_DEVERR_NONE = 0, SKINNY_DEVERR_TIMEOUT = 1 };
@@ -303,6 +317,9 @@ __device__ __forceinline__ void fence_mbar_init() {
 }
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
@@ -336,6 +353,55 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (mbar_try_wait(bar, parity)) return true;
   if (err) atomicExch(err, SKINNY_DEVERR_TIMEOUT);
   return false;
+}
+
+template <typename T>
+__device__ __forceinline__ T tzero() {
+  return T(0);
+}
+template <>
+__device__ __forceinline__ c32 tzero<c32>() {
+  return {0.f, 0.f};
+}
+template <>
+__device__ __forceinline__ c64 tzero<c64>() {
+  return {0.0, 0.0};
+}
+template <>
+__device__ __forceinline__ c32h tzero<c32h>() {
+  return {0.f, 0.f};
+}
+template <>
+__device__ __forceinline__ c64h tzero<c64h>() {
+  return {0.0, 0.0};
+}
+
+// L2-coherent loads of partials written by other CTAs (L1 is not coherent across SMs).
+__device__ __forceinline__ float ldcg(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ c32 ldcg(const c32* p) {
+  float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ c64 ldcg(const c64* p) {
+  double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ c32h ldcg(const c32h* p) {
+  float2 v = __ldcg(reinterpret_cast<const float2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ c64h ldcg(const c64h* p) {
+  double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ dd ldcg(const dd* p) {
+  double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ zdd ldcg(const zdd* p) {
+  const double2 a = __ldcg(reinterpret_cast<const double2*>(p)), b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+  return {{a.x, a.y}, {b.x, b.y}};
 }
 
 __host__ __device__ constexpr int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -12,6 +12,5 @@ namespace skinny {
 template skinny_status tsmttsm_plan<double, double>(const DeviceInfo&, int64_t, int64_t, int64_t,
                                                     const void*, int64_t, const void*, int64_t, bool,
                                                     const LaunchOpts&, TsmttsmPlan&);
-template skinny_status tsmttsm_dispatch<double, double>(int, int, const TsmttsmArgs<double>&, dim3,
-                                                        int, cudaStream_t);
+template skinny_status tsmttsm_dispatch<double, double>(const TsmttsmPlan&, const TsmttsmArgs<double>&, cudaStream_t);
 }  // namespace skinny

@@ -82,10 +82,10 @@ inline bool ensure_smem_attr(K kernel, int bytes, SmemAttr& done) {
 }
 
 // ----------------------------------------------------------------------------------- TSMTTSM
-template <typename T, typename Acc, int TM, int TN>
+template <typename T, typename Acc, int TM, int TN, bool VEC>
 skinny_status tsmttsm_launch_tile(const TsmttsmArgs<T>& a, dim3 grid, int smem, cudaStream_t st) {
   static SmemAttr attr;
-  auto kern = tsmttsm_kernel<T, Acc, TM, TN>;
+  auto kern = tsmttsm_kernel<T, Acc, TM, TN, VEC>;
   ensure_smem_attr(kern, smem, attr);
   kern<<<grid, TSMTTSM_THREADS, smem, st>>>(a);
   count_launch();
@@ -101,15 +101,30 @@ skinny_status tsmttsm_launch_tile(const TsmttsmArgs<T>& a, dim3 grid, int smem, 
 // 32 of 16 bytes, 8 of 32 bytes (complex double-double)
 template <typename Acc>
 constexpr int tile_cap() {
-  return sizeof(Acc) >= 32 ? 8 : (int)(128 / (sizeof(Acc) / 4));
+  return sizeof(Acc) >= 32 ? 8 : (int)(128 / (sizeof(Acc) / 4) < 64 ? 128 / (sizeof(Acc) / 4) : 64);
 }
+struct TsmttsmPlan {
+  int tm, tn, rows, stages, grid, groups, smem, bulk, vec;
+  int64_t ntiles, lda_s, ldb_s;
+  int entries;  // of a CTA's partial: its cells' register tiles
+  // workspace bytes of a grid of nb CTAs (fewer than planned: less)
+  template <typename Acc>
+  size_t partials(int nb) const {
+    return (groups > 1 ? (size_t)nb * groups * TSMTTSM_THREADS * tm * tn : (size_t)finish_entries<Acc>(nb, entries)) *
+           sizeof(Acc);
+  }
+};
 
 template <typename T, typename Acc>
-skinny_status tsmttsm_dispatch(int tm, int tn, const TsmttsmArgs<T>& a, dim3 grid, int smem,
-                               cudaStream_t st) {
-#define SK_TILE(X, Y)                                                                   \
-  if constexpr (X * Y <= tile_cap<Acc>() && X * Y <= 64)                                \
-    if (tm == X && tn == Y) return tsmttsm_launch_tile<T, Acc, X, Y>(a, grid, smem, st);
+skinny_status tsmttsm_dispatch(const TsmttsmPlan& pl, const TsmttsmArgs<T>& a, cudaStream_t st) {
+  const dim3 grid(pl.grid, pl.groups);
+#define SK_TILE(X, Y)                                                                             \
+  if constexpr (X * Y <= tile_cap<Acc>())                                                         \
+    if (pl.tm == X && pl.tn == Y) {                                                               \
+      if constexpr (std::is_same<T, float>::value && std::is_same<Acc, float>::value && X * Y > 1) \
+        if (pl.vec) return tsmttsm_launch_tile<T, Acc, X, Y, true>(a, grid, pl.smem, st);         \
+      return tsmttsm_launch_tile<T, Acc, X, Y, false>(a, grid, pl.smem, st);                      \
+    }
   SK_TILE(1, 1) SK_TILE(1, 2) SK_TILE(1, 4) SK_TILE(1, 8)
   SK_TILE(2, 1) SK_TILE(2, 2) SK_TILE(2, 4) SK_TILE(2, 8)
   SK_TILE(4, 1) SK_TILE(4, 2) SK_TILE(4, 4) SK_TILE(4, 8)
@@ -119,21 +134,70 @@ skinny_status tsmttsm_dispatch(int tm, int tn, const TsmttsmArgs<T>& a, dim3 gri
   return SKINNY_UNSUPPORTED;
 }
 
-struct TsmttsmPlan {
-  int tm, tn, rows, stages, grid, groups, smem, bulk;
-  int64_t ntiles, lda_s, ldb_s;
-  size_t partial_bytes;
-};
+// Clocks one SM takes for `rows` rows with TM x TN cells, and for its reduction (model).  FP64-pipe
+// types: a warp instruction holds the pipe of its SM partition (one of 4) for ~68 clocks, so the
+// time is the busiest partition's warps times the tile, padding included, and reducing the CTA
+// costs about 1.5 more tiles per thread.  FP32: 128 FMAs per clock and SM against shared-memory
+// wavefronts (one per 16-byte vector load of a warp, two counted), with HBM below both.
+template <typename T, typename Acc>
+double tsmttsm_tile_cost(int64_t M, int64_t N, int tm, int tn, int64_t cells, bool vec, double rows, double row_bytes) {
+  const int RS = (int)(TSMTTSM_THREADS / cells);
+  const int warps = (int)((cells * RS + 31) / 32), busiest = (warps + 3) / 4;
+  const int t = tm * tn;
+  if (!fp32_sums<Acc>()) {
+    const double macs = std::is_same<Acc, zdd>::value ? 32 : std::is_same<Acc, dd>::value ? 8 : sizeof(Acc) / 4;
+    const double adds = std::is_same<Acc, zdd>::value ? 40 : std::is_same<Acc, dd>::value ? 20 : sizeof(Acc) / 8;
+    return 68.0 * busiest * t * (macs * (sizeof(Acc) == 8 ? 0.5 : 1.0) * rows / RS + 1.5 * adds);
+  }
+  const double flops = std::is_same<Acc, float>::value ? 1 : 4;
+  const double fma = busiest * t * flops;
+  const double lds = warps * (vec ? 2.0 * ((tm + 3) / 4 + (tn + 3) / 4) : 1.5 * (tm + tn));
+  const double step = std::max(fma, lds) + 0.3 * std::min(fma, lds) + 4.0 * busiest;
+  return std::max(step / RS, row_bytes / 44.0) * rows + t * 8.0 * busiest;
+}
 
 template <typename T, typename Acc>
 skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t K, const void* A,
                            int64_t lda, const void* B, int64_t ldb, bool gram, const LaunchOpts& o,
                            TsmttsmPlan& pl) {
   const int cap = tile_cap<Acc>();
-  int tm = pow2ceil(M) < 8 ? pow2ceil(M) : 8;
-  int tn = pow2ceil(N) < 8 ? pow2ceil(N) : 8;
-  while (tm * tn > cap) (tm >= tn ? tm : tn) /= 2;
-  const int64_t Gall = ((M + tm - 1) / tm) * ((N + tn - 1) / tn);
+  const int64_t s = sizeof(T);
+  const bool aligned = ((uintptr_t)A % 16 == 0) && (gram || (uintptr_t)B % 16 == 0);
+  const bool dense = lda <= 2 * M + 16 && (gram || ldb <= 2 * N + 16);
+  // shared row strides: ld when bulk-copied, dense (M / N) when loaded by threads
+  const int64_t row_bytes_bulk = (lda + (gram ? 0 : ldb)) * s;
+  const int64_t row_bytes_dense = (M + (gram ? 0 : N)) * s;
+  const int64_t rb = (aligned && dense) ? row_bytes_bulk : row_bytes_dense;
+  const int64_t las = aligned && dense ? lda : M, lbs = gram ? las : (aligned && dense ? ldb : N);
+  pl.vec = std::is_same<T, float>::value && las % 4 == 0 && lbs % 4 == 0;
+
+  // the tile: the cheapest one whose cells fit one group of threads; beyond, the largest
+  const double sm_rows = (double)K / (dev.sms > 0 ? dev.sms : 1);
+  double best = -1.0;
+  pl.tm = pl.tn = 0;
+  const int pm = std::min(pow2ceil(M), 8), pn = std::min(pow2ceil(N), 8);
+  for (int tm = 1; tm <= pm; tm *= 2)
+    for (int tn = 1; tn <= pn; tn *= 2) {
+      if (tm * tn > cap || (gram && tm != tn)) continue;
+      if (sizeof(Acc) == 8 && tm * tn > 16) continue;
+      const int64_t gm = (M + tm - 1) / tm, gn = (N + tn - 1) / tn;
+      const int64_t cells = gram ? gm * (gm + 1) / 2 : gm * gn;
+      if (cells > TSMTTSM_THREADS) continue;
+      const double c = tsmttsm_tile_cost<T, Acc>(M, N, tm, tn, cells, pl.vec != 0, sm_rows, (double)rb);
+      if (best < 0.0 || c < best) {
+        best = c;
+        pl.tm = tm;
+        pl.tn = tn;
+      }
+    }
+  if (best < 0.0) {
+    pl.tm = pm;
+    pl.tn = pn;
+    while (pl.tm * pl.tn > cap) (pl.tm >= pl.tn ? pl.tm : pl.tn) /= 2;
+  }
+  const int tm = pl.tm, tn = pl.tn;
+  const int64_t gm = (M + tm - 1) / tm, gn = (N + tn - 1) / tn;
+  const int64_t Gall = gram && tm == tn ? gm * (gm + 1) / 2 : gm * gn;
   const int64_t groups = (Gall + TSMTTSM_THREADS - 1) / TSMTTSM_THREADS;
   if (groups > 64) {  // one ticket counter per group in the 256-byte counter block
     set_error("tsmttsm: M, N too large for the CUDA-core kernel");
@@ -141,71 +205,78 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
   }
   const int64_t G = Gall < TSMTTSM_THREADS ? Gall : TSMTTSM_THREADS;
   const int RS = (int)(TSMTTSM_THREADS / G);
-  const int64_t s = sizeof(T);
-  const bool aligned = ((uintptr_t)A % 16 == 0) && (gram || (uintptr_t)B % 16 == 0);
-  const bool dense = lda <= 2 * M + 16 && (gram || ldb <= 2 * N + 16);
-  // shared row strides: ld when bulk-copied, dense (M / N) when loaded by threads
-  int64_t row_bytes_bulk = (lda + (gram ? 0 : ldb)) * s;
-  int64_t row_bytes_dense = (M + (gram ? 0 : N)) * s;
+  // as many CTAs as stay resident once an SM has rows enough to repay their reductions
+  int bps = o.blocks_per_sm;
+  if (bps <= 0) {
+    bps = tsmttsm_ctas<Acc>(tm * tn);
+    if (sm_rows < 256.0) bps = 1;
+  }
+  const int64_t ctas = (int64_t)std::max(dev.sms, 1) * bps;
   int rows = o.rows_per_tile;
-  int64_t rb = (aligned && dense) ? row_bytes_bulk : row_bytes_dense;
   if (rows <= 0) {
-    int64_t r = 16384 / rb;
-    rows = 16;
-    while (rows * 2 <= r && rows < 1024) rows *= 2;
+    // FP64-pipe types: 16 KB.  FP32: a third of the CTA's shared memory, for a tile of 16 KB is
+    // only a few rows per thread and the hand-offs show (13 x 7, 3.4e6 rows: 102 us; 69 with 32 KB)
+    const int64_t most = fp32_sums<Acc>() ? (int64_t)208 * 1024 / bps / 3 - 256 : 16384;
+    rows = (int)std::max<int64_t>(16, std::min<int64_t>(1024, most / rb / 16 * 16));
+    // the same whole number of tiles for every CTA (rows are handed out in 16s), at least two
+    // each where K allows, so that copies and sums overlap
+    const int64_t per_cta = std::max<int64_t>((K + ctas - 1) / ctas, 1);
+    const int64_t n = std::max<int64_t>((per_cta + rows - 1) / rows, per_cta >= 64 ? 2 : 1);
+    rows = (int)std::min<int64_t>(rows, round_up((per_cta + n - 1) / n, 16));
   }
   rows = (int)round_up(rows < RS ? RS : rows, 16);
-  const int64_t stage_a = round_up(rows * (aligned && dense ? lda : M) * s, 128);
-  const int64_t stage_b = gram ? 0 : round_up(rows * (aligned && dense ? ldb : N) * s, 128);
+  const int64_t stage_a = round_up(rows * las * s, 128);
+  const int64_t stage_b = gram ? 0 : round_up(rows * lbs * s, 128);
   const int64_t stage = stage_a + stage_b;
   const bool bulk = aligned && dense && stage <= 65536 && K > rows;
   const int64_t budget = (int64_t)dev.smem_optin - SMEM_HEADER - 1024;
-  int stages = (int)std::min<int64_t>(8, (160 * 1024) / std::max<int64_t>(stage, 1));
+  int stages = (int)std::min<int64_t>(TSMTTSM_MAX_STAGES, (208 * 1024 / bps) / std::max<int64_t>(stage, 1));
   if (stages < 2) stages = 2;
   if (stages * stage > budget) stages = (int)(budget / stage);
   if (stages < 1) {
     set_error("tsmttsm: row tile does not fit in shared memory");
     return SKINNY_UNSUPPORTED;
   }
-  pl.tm = tm;
-  pl.tn = tn;
   pl.rows = rows;
   pl.stages = stages;
   pl.bulk = bulk;
   pl.lda_s = bulk ? lda : M;
   pl.ldb_s = gram ? pl.lda_s : (bulk ? ldb : N);
+  if (!bulk) pl.vec = std::is_same<T, float>::value && pl.lda_s % 4 == 0 && pl.ldb_s % 4 == 0;
   pl.ntiles = (K + rows - 1) / rows;
-  int64_t smem = SMEM_HEADER + stages * stage;
-  const int64_t red = (int64_t)(M * N + TSMTTSM_THREADS) * sizeof(Acc);
-  if (red + SMEM_HEADER <= budget && smem < SMEM_HEADER + red) smem = SMEM_HEADER + red;
-  pl.smem = (int)smem;
-  const int bps = o.blocks_per_sm > 0 ? o.blocks_per_sm : 1;
-  int64_t grid = (int64_t)dev.sms * bps;
+  const int nslots = G < 32 && (G & (G - 1)) == 0 ? TSMTTSM_THREADS / 32 : RS;
+  const int64_t E = G * tm * tn;
+  const int64_t red = std::max<int64_t>(nslots > 1 ? nslots * E : 0, TSMTTSM_THREADS) * (int64_t)sizeof(Acc);
+  pl.smem = (int)(SMEM_HEADER + std::max(stages * stage + SMEM_SLACK, red));
+  int64_t grid = ctas;
   if (grid > pl.ntiles) grid = pl.ntiles;
   if (grid < 1) grid = 1;
   pl.grid = (int)grid;
   pl.groups = (int)groups;
-  pl.partial_bytes = (size_t)grid * (size_t)(M * N) * sizeof(Acc);
+  pl.entries = (int)E;
   return SKINNY_OK;
 }
 
 // ----------------------------------------------------------------- TSMTTSM, narrow products
-// Register-tile entries a thread of the row-streaming kernel may hold: 64 for 4- and 8-byte
-// accumulators (FP64 8 x 8), 16 for 16-byte ones (complex FP64, double-double), 4 for 32-byte
-// ones (complex double-double).
+// Register-tile entries a thread of the row-streaming kernel may hold: 64 for sums on the FP32 pipe
+// (8 x 8), 16 for FP64 (8 x 8 on the ring kernel: 11.1 us against 14.6 at 2^14 rows, the same at
+// 2^20; 7 x 7 116 us against 143 at 1.2e6 rows), 16 for other 16-byte accumulators (complex FP64, double-double), 4 for
+// 32-byte ones (complex double-double).
 template <typename Acc>
 constexpr int rows_cap() {
-  return sizeof(Acc) <= 8 ? 64 : (sizeof(Acc) <= 16 ? 16 : 4);
+  return fp32_sums<Acc>() ? 64 : (sizeof(Acc) <= 16 ? 16 : 4);
 }
 
 // The row-streaming kernel takes a product when both padded widths are <= 8 and their tile fits
-// rows_cap; an autotuned row-tile size asks for the ring kernel instead.
+// rows_cap; an autotuned row-tile size asks for the ring kernel instead.  FP32-pipe tiles above 16
+// entries stay with it below 2^20 rows (8 x 8 FP32: 5.1 us against 7.6 at 2^14 rows, 10.8 against
+// 12.3 at 2^18, the same at 2^20; 70 against 55 at 2^22: 64 sums a thread leave few loads in flight).
 template <typename T, typename Acc>
-bool rows_eligible(int64_t M, int64_t N, bool gram, const LaunchOpts& o) {
+bool rows_eligible(int64_t M, int64_t N, int64_t K, bool gram, const LaunchOpts& o) {
   if (o.rows_per_tile > 0 || M < 1 || N < 1 || M > 8 || N > 8) return false;
   int tm = pow2ceil(M), tn = pow2ceil(N);
   if (gram) tm = tn = std::max(tm, tn);
-  return tm * tn <= rows_cap<Acc>();
+  return tm * tn <= rows_cap<Acc>() && (tm * tn <= 16 || K < (1 << 20));
 }
 
 template <typename T, typename Acc, int TM, int TN>
@@ -221,10 +292,16 @@ skinny_status tsmttsm_rows_launch(RowsArgs<T>& a, const DeviceInfo& dev, Workspa
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ROWS_THREADS, 0);
     if (occ < 1) occ = 1;
     if (bps_opt > 0 && bps_opt < occ) occ = bps_opt;
+    // FP64-pipe types: at least 4 rows per thread, or reducing the extra CTAs costs more than they
+    // save (FP64 4 x 4, 2^18 rows: 21.7 us with full occupancy, 16.0 with 2 CTAs per SM)
+    if (!fp32_sums<Acc>() && bps_opt <= 0) {
+      const int64_t most = (a.K + (int64_t)dev.sms * ROWS_THREADS * 4 - 1) / ((int64_t)dev.sms * ROWS_THREADS * 4);
+      if (most < occ) occ = (int)std::max<int64_t>(most, 1);
+    }
     const int64_t per_cta = (int64_t)ROWS_THREADS * U;
     int64_t grid = std::min<int64_t>((int64_t)dev.sms * occ, (a.K + per_cta - 1) / per_cta);
     if (grid < 1) grid = 1;
-    skinny_status s = workspace_ensure(ws, (size_t)grid * (size_t)(a.M * a.N) * sizeof(Acc), st);
+    skinny_status s = workspace_ensure(ws, (size_t)finish_entries<Acc>((int)grid, TM * TN) * sizeof(Acc), st);
     if (s != SKINNY_OK) return s;
     a.partials = ws.partials;
     a.counter = ws.counter;
@@ -283,12 +360,12 @@ skinny_status tsmttsm_run(const DeviceInfo& dev, Workspace& ws, int* err, cudaSt
                           const T* B, int64_t ldb, T beta, bool beta_zero, T* C, int64_t ldc,
                           const LaunchOpts& o) {
   const bool gram = (A == B) && (lda == ldb) && (M == N);
-  if (rows_eligible<T, Acc>(M, N, gram, o))
+  if (rows_eligible<T, Acc>(M, N, K, gram, o))
     return tsmttsm_rows_run<T, Acc>(dev, ws, st, M, N, K, A, lda, alpha, B, ldb, beta, beta_zero, C, ldc, gram, o);
   TsmttsmPlan pl;
   skinny_status s = tsmttsm_plan<T, Acc>(dev, M, N, K, A, lda, B, ldb, gram, o, pl);
   if (s != SKINNY_OK) return s;
-  s = workspace_ensure(ws, pl.partial_bytes, st);
+  s = workspace_ensure(ws, pl.partials<Acc>(pl.grid), st);
   if (s != SKINNY_OK) return s;
   TsmttsmArgs<T> a;
   a.A = A;
@@ -313,12 +390,11 @@ skinny_status tsmttsm_run(const DeviceInfo& dev, Workspace& ws, int* err, cudaSt
   const int64_t sz = sizeof(T);
   a.bytes_a = (uint32_t)round_up(pl.rows * pl.lda_s * sz, 128);
   a.bytes_b = gram ? 0u : (uint32_t)round_up(pl.rows * pl.ldb_s * sz, 128);
-  a.smem_avail = (uint32_t)(pl.smem - SMEM_HEADER);
   a.partials = ws.partials;
   a.counter = ws.counter;
   a.err = err;
   a.polls = dev.wait_polls;
-  return tsmttsm_dispatch<T, Acc>(pl.tm, pl.tn, a, dim3(pl.grid, pl.groups), pl.smem, st);
+  return tsmttsm_dispatch<T, Acc>(pl, a, st);
 }
 
 // -------------------------------------------------------------------------------------- TSMM

@@ -24,8 +24,8 @@ extern template skinny_status tsmttsm_plan<double, double>(const DeviceInfo&, in
                                                            int64_t, const void*, int64_t,
                                                            const void*, int64_t, bool,
                                                            const LaunchOpts&, TsmttsmPlan&);
-extern template skinny_status tsmttsm_dispatch<double, double>(int, int, const TsmttsmArgs<double>&,
-                                                               dim3, int, cudaStream_t);
+extern template skinny_status tsmttsm_dispatch<double, double>(const TsmttsmPlan&, const TsmttsmArgs<double>&,
+                                                               cudaStream_t);
 
 constexpr size_t kStaticCounterBytes = 256;            // 64 ticket counters, cleared per call
 constexpr size_t kStaticErrOffset = 256;               // device error word (bounded waits)
@@ -89,7 +89,6 @@ extern "C" skinny_status skinny_tsmttsm_d_static(int64_t M, int64_t N, int64_t K
     set_error("static TSMTTSM: M*N exceeds the static scratch (at most 1048576 entries of C)");
     return SKINNY_BAD_ARG;
   }
-  const size_t per_cta = (size_t)M * (size_t)N * sizeof(double);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
@@ -104,8 +103,7 @@ extern "C" skinny_status skinny_tsmttsm_d_static(int64_t M, int64_t N, int64_t K
   TsmttsmPlan pl;
   s = tsmttsm_plan<double, double>(sd->info, M, N, K, A, lda, B, ldb, gram, LaunchOpts{}, pl);
   if (s != SKINNY_OK) return s;
-  const int64_t max_grid = (int64_t)(kStaticPartialBytes / per_cta);
-  if (pl.grid > max_grid) pl.grid = (int)max_grid;  // fewer CTAs so the partials fit
+  while (pl.grid > 1 && pl.partials<double>(pl.grid) > kStaticPartialBytes) pl.grid--;  // until the partials fit
 
   cudaStream_t st = (cudaStream_t)stream;
   // the ticket counters must start at zero; an earlier call that timed out leaves them behind
@@ -136,12 +134,11 @@ extern "C" skinny_status skinny_tsmttsm_d_static(int64_t M, int64_t N, int64_t K
   a.ntiles = pl.ntiles;
   a.bytes_a = (uint32_t)round_up(pl.rows * pl.lda_s * (int64_t)sizeof(double), 128);
   a.bytes_b = gram ? 0u : (uint32_t)round_up(pl.rows * pl.ldb_s * (int64_t)sizeof(double), 128);
-  a.smem_avail = (uint32_t)(pl.smem - SMEM_HEADER);
   a.partials = sd->base + kStaticHeaderBytes;
   a.counter = reinterpret_cast<unsigned*>(sd->base);
   a.err = reinterpret_cast<int*>(sd->base + kStaticErrOffset);
   a.polls = kWaitPolls;
-  return tsmttsm_dispatch<double, double>(pl.tm, pl.tn, a, dim3(pl.grid, pl.groups), pl.smem, st);
+  return tsmttsm_dispatch<double, double>(pl, a, st);
 }
 
 extern "C" skinny_status skinny_tsmttsm_d_static_check(void* stream) {

@@ -1,5 +1,5 @@
 // tsmttsm_rows.cuh -- TSMTTSM on CUDA cores for narrow products (padded M x N up to 16 entries, or
-// 8 x 8 in FP64): C(MxN) = alpha * A^T B + beta * C.
+// up to 8 x 8 on the FP32 pipe): C(MxN) = alpha * A^T B + beta * C.
 //
 // Replaces, for these widths, the reference's GENV3X / SPECSMALL blockProductKernel +
 // deviceReduce pairs (tsmttsm/genv3x.cuh:29-81, specsmall.cuh:28-90), which on GB300 stream
@@ -14,14 +14,15 @@
 //     leading dimensions allow it.  Gram mode (A == B) reads A only.
 //   * Rows are spread grid-stride over a grid of several CTAs per SM; no shared-memory staging,
 //     no barriers in the streaming loop.
-//   * Reduction: butterfly warp shuffles, the warps of a CTA in warp order through shared memory,
-//     one partial per CTA in the workspace, and the last CTA to take the ticket sums the CTA
-//     partials in CTA order (slices of the CTA range, then the slices in order) and applies
-//     alpha / beta.  The result is deterministic; the ticket is reset for the next launch.
+//   * Reduction (reduce.cuh): halving warp shuffles, the warps of a CTA in a shared-memory tree,
+//     one partial per CTA in the workspace, summed by ticket on one or two levels by the last CTAs,
+//     which apply alpha / beta.  The result is deterministic; the tickets are reset for the next
+//     launch.
 #pragma once
 #include <type_traits>
 
 #include "common.cuh"
+#include "reduce.cuh"
 #include "tsmttsm.cuh"
 
 namespace skinny {
@@ -68,11 +69,9 @@ __global__ void __launch_bounds__(ROWS_THREADS) tsmttsm_rows_kernel(const RowsAr
   const int M = p.M, N = p.N;
   const bool gram = p.gram != 0;
 
-  Acc acc[TM][TN];
+  Acc acc[TMN];
 #pragma unroll
-  for (int x = 0; x < TM; x++)
-#pragma unroll
-    for (int y = 0; y < TN; y++) acc[x][y] = O::zero();
+  for (int i = 0; i < TMN; i++) acc[i] = O::zero();
 
   const int64_t stride = (int64_t)gridDim.x * NT * U;
   for (int64_t base = (int64_t)blockIdx.x * NT * U + tid; base < p.K; base += stride) {
@@ -96,62 +95,31 @@ __global__ void __launch_bounds__(ROWS_THREADS) tsmttsm_rows_kernel(const RowsAr
           } else {
             bv = b[j][y];  // Gram mode is never planned with TN > TM
           }
-          acc[x][y] = O::mac(acc[x][y], a[j][x], bv);
+          acc[x * TN + y] = O::mac(acc[x * TN + y], a[j][x], bv);
         }
   }
 
-  // ---- CTA reduction: warp butterflies, then the warps in order ------------------------------
-#pragma unroll
-  for (int x = 0; x < TM; x++)
-#pragma unroll
-    for (int y = 0; y < TN; y++)
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) acc[x][y] = O::add(acc[x][y], O::shfl_xor(acc[x][y], o));
-  __shared__ Acc wsum[NW][TMN];
+  // ---- CTA reduction: halving shuffles, the warps in a tree, then the CTAs --------------------
+  __shared__ Acc wsum[NW * TMN];
   __shared__ Acc slices[NT];
-  __shared__ int s_last;
-  if (lane == 0) {
+  __shared__ int s_flag;
+  int e0 = 0, ne = TMN;
+  bool owner = true;
+  warp_halve<O, Acc, TMN>(acc, 1, lane, e0, ne, owner);
+  if (owner) {
 #pragma unroll
-    for (int x = 0; x < TM; x++)
-#pragma unroll
-      for (int y = 0; y < TN; y++) wsum[warp][y * TM + x] = acc[x][y];
+    for (int i = 0; i < (TMN + 31) / 32; i++) wsum[warp * TMN + e0 + i] = acc[i];
   }
   __syncthreads();
-  const int MN = M * N;
+  slot_tree<O, Acc, NT>(wsum, NW, TMN);
   Acc* part = reinterpret_cast<Acc*>(p.partials);
-  if (tid < MN) {
-    const int m = tid % M, n = tid / M;
-    Acc s = wsum[0][n * TM + m];
-#pragma unroll
-    for (int w = 1; w < NW; w++) s = O::add(s, wsum[w][n * TM + m]);
-    part[(size_t)blockIdx.x * MN + tid] = s;
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = (atomicAdd(p.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-
-  // ---- last CTA: the CTA partials in CTA order (P slices of the CTA range, then the slices) ---
-  const int nb = gridDim.x;
-  const int P = NT / MN;  // MN <= 64, so P >= 4
-  const int e = tid % MN, j = tid / MN;
-  if (j < P) {
-    Acc sum = O::zero();
-    const int b0 = (int)((int64_t)nb * j / P), b1 = (int)((int64_t)nb * (j + 1) / P);
-    for (int b = b0; b < b1; b++) sum = O::add(sum, ldcg(&part[(size_t)b * MN + e]));
-    slices[j * MN + e] = sum;
-  }
-  __syncthreads();
-  if (tid < MN) {
-    Acc s = slices[tid];
-    for (int q = 1; q < P; q++) s = O::add(s, slices[q * MN + tid]);
-    const int m = tid % M, n = tid / M;
+  if (tid < TMN) part[(size_t)blockIdx.x * TMN + tid] = wsum[tid];
+  finish_partials<O, Acc, NT>(part, p.counter, TMN, true, slices, &s_flag, [&](int e, Acc s) {
+    const int m = e / TN, n = e % TN;
+    if (m >= M || n >= N) return;
     T* c = p.C + (int64_t)n * p.ldc + m;
     *c = O::finish(s, p.alpha, p.beta, p.beta_zero != 0, c);
-  }
-  if (tid == 0) *p.counter = 0u;
+  });
 }
 
 }  // namespace skinny
