@@ -12,6 +12,7 @@
 
 #include "skinny.h"
 #include "tsmm.cuh"
+#include "tsmm_tile.cuh"
 #include "tsmttsm.cuh"
 #include "tsmttsm_rows.cuh"
 
@@ -422,6 +423,57 @@ skinny_status tsmm_launch_tile(const TsmmArgs<T>& a, int bps, int sms, int smem,
   return SKINNY_OK;
 }
 
+template <typename T, int R>
+skinny_status tsmm_tile_launch(const TsmmTileArgs<T>& a, int bps, int sms, int smem, cudaStream_t st) {
+  static SmemAttr attr;
+  auto kern = tsmm_tile_kernel<T, R>;
+  if (!ensure_smem_attr(kern, smem, attr)) return SKINNY_DEVICE_ERROR;
+  int occ = smem <= 112 * 1024 ? 2 : 1;  // what the registers and the shared memory of an SM hold
+  if (bps > 0 && bps < occ) occ = bps;
+  const int64_t rows = TSMM_THREADS / a.t.gn * R;
+  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * occ, (a.t.K + rows - 1) / rows));
+  kern<<<(int)grid, TSMM_THREADS, smem, st>>>(a);
+  count_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error(std::string("tsmm launch: ") + cudaGetErrorString(e));
+    return SKINNY_DEVICE_ERROR;
+  }
+  return SKINNY_OK;
+}
+
+// The tiled kernel for float and complex float; false: the shape is left to tsmm_kernel (at most 4
+// columns in and out, which that streams at 0.75 of HBM rate, more than 128 outputs, or a tile that
+// does not fit).  Rows per thread: 8 where the FMA pipe is near (more than 16 columns of output), 4
+// otherwise, fewer while a CTA's ring is above 110 KB (two CTAs per SM) or SMs would go without rows.
+template <typename T>
+bool tsmm_tile_run(const DeviceInfo& dev, cudaStream_t st, const TsmmArgs<T>& t, const LaunchOpts& o, skinny_status& s) {
+  constexpr int V = 16 / (int)sizeof(T);
+  const int M = t.M, N = t.N;
+  if (M * (int)sizeof(T) <= 16 && N * (int)sizeof(T) <= 16) return false;
+  TsmmTileArgs<T> a;
+  a.t = t;
+  a.t.gn = pow2ceil((N + V - 1) / V);
+  a.t.np = a.t.gn * V;
+  if (a.t.gn > 32) return false;
+  const int chunks = (M + V - 1) / V;
+  a.stride = (chunks % 2 ? chunks : chunks + 1) * V;
+  a.vec_a = M % V == 0 && t.lda % V == 0 && (uintptr_t)t.A % 16 == 0;
+  a.vec_c = t.ldc % V == 0 && (uintptr_t)t.C % 16 == 0;
+  const int64_t bs = (int64_t)M * a.t.np * sizeof(T);
+  const int RP = TSMM_THREADS / a.t.gn;
+  auto smem = [&](int R) { return bs + (int64_t)TSMM_TILE_STAGES * RP * R * a.stride * sizeof(T); };
+  int R = N * (int)sizeof(T) > 64 ? 8 : 4;
+  while (R > 1 && (smem(R) > 110 * 1024 || (t.K + RP * R - 1) / (RP * R) < 2 * dev.sms)) R /= 2;
+  if (smem(R) > dev.smem_optin - 1024) return false;
+  const int sm = (int)smem(R), b = o.blocks_per_sm;
+  s = R == 8   ? tsmm_tile_launch<T, 8>(a, b, dev.sms, sm, st)
+      : R == 4 ? tsmm_tile_launch<T, 4>(a, b, dev.sms, sm, st)
+      : R == 2 ? tsmm_tile_launch<T, 2>(a, b, dev.sms, sm, st)
+               : tsmm_tile_launch<T, 1>(a, b, dev.sms, sm, st);
+  return true;
+}
+
 template <typename T, typename Acc>
 skinny_status tsmm_run(const DeviceInfo& dev, cudaStream_t st, int64_t M, int64_t N, int64_t K,
                        const T* A, int64_t lda, T alpha, const T* B, int64_t ldb, T beta,
@@ -456,6 +508,10 @@ skinny_status tsmm_run(const DeviceInfo& dev, cudaStream_t st, int64_t M, int64_
   a.fold = (const void*)A == (const void*)C && lda == ldc && M == N && !beta_zero && sizeof(Acc) == sizeof(T);
   a.gn = gn;
   a.np = np;
+  if constexpr (std::is_same<T, Acc>::value && (std::is_same<T, float>::value || std::is_same<T, c32>::value)) {
+    skinny_status s;
+    if (tsmm_tile_run<T>(dev, st, a, o, s)) return s;
+  }
   const int sm = (int)(smem < 16 ? 16 : smem);
   // narrow rows (M <= 4, a few outputs per thread): 4 rows per thread and step
   // (32-byte accumulators: one row per thread and step)
