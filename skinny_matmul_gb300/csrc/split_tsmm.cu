@@ -18,20 +18,21 @@
 //     leading level).  |D_L| <= 2^14 MP (L - 2) (the top digit is at most 64 in magnitude): exact
 //     in the FP32 TMEM accumulators.
 //   * Epilogue: V = sum_L D_L 2^(8(9-L)) (|V| < 2^74) is formed as a 64-bit integer W = V / 2^12
-//     (level_window), rounded to a double (integer instructions, or the FP64 pipe's conversion
-//     when there is no beta*C) and scaled by 2^(e_r + f_n - 2100) in the exponent field; beta*C
+//     (level_window), rounded to a double (by integer instructions or the FP64 pipe's conversion) and scaled by 2^(e_r + f_n - 2100) in the exponent field; beta*C
 //     is one FMA.
-//   * Warp roles, hand-offs through mbarriers, no CTA-wide barrier while streaming (16 warps):
+//   * Warp roles, hand-offs through mbarriers, no CTA-wide barrier while streaming (16 or 24 warps):
 //       slicers     (8 warps, two threads per row) read the FP64 values of a 128-row tile (the
 //                   next tile's are loaded right after a tile is sliced), take the row exponent,
 //                   and write the digit planes into an A' stage; warp 0 then issues the tile's
 //                   MMAs (one elected lane): per block of NB output columns, 8 MP / 16 MMAs into
 //                   one of 2 or 4 TMEM accumulator sets, so that a block's epilogue overlaps the
 //                   next blocks' MMAs;
-//       epilogue    (8 warps: 2 groups of one warp per TMEM lane quadrant) convert the level
-//                   sums; the groups take chunks of 8 output columns in turn; old C values are
-//                   prefetched chunk by chunk (cp.async) into a shared-memory ring per group,
-//                   several chunks ahead.
+//       epilogue    (2 or 4 groups of one warp per TMEM lane quadrant) convert the level sums; the
+//                   groups take chunks of 4 output columns in turn; old C values are prefetched
+//                   chunk by chunk (cp.async) into a shared-memory ring per group, several chunks
+//                   ahead.
+//     Ring positions and parities are counters, not remainders: dividing the tile number by the
+//     run-time ring sizes took a quarter of the instructions of a 16 x 16 tile.
 //     Every wait is bounded; a wait that runs out sets the error word and every role stops at its
 //     next wait (C is then incomplete).
 //   * In place with M == N, beta is folded into the diagonal of alpha*B before slicing
@@ -51,17 +52,16 @@ namespace stsmm {
 
 constexpr int ROWS = 128;
 constexpr int DIGITS = 8;
-constexpr int THREADS = 512;  // 16 warps: four per SM sub-partition, 128 registers
-// Warp roles: 8 slicer warps (two threads per row; warp 0 issues the MMAs) and 8 epilogue warps
-// (two groups of one warp per TMEM lane quadrant).  Measured and dropped at MP = 16: 4 slicer
-// warps (one thread per row) with 12 epilogue warps -- three groups split blocks of 2 or 4 chunks
-// unevenly, and the slicers fell behind (real 8 x 32 3.76 -> 4.60 ms, 16 x 16 1.14 -> 1.25 ms).
-template <int MP>
-__host__ __device__ constexpr int slicer_warps() { return 8; }
-template <int MP>
-__host__ __device__ constexpr int epi_groups() { return (16 - slicer_warps<MP>()) / 4; }
+// Warp roles: 8 slicer warps (two threads per row; warp 0 also issues the MMAs) and NW - 8 epilogue
+// warps in groups of one per TMEM lane quadrant.  NW = 16 warps of 128 registers; contraction width
+// 16 with more than 16 output columns, where the epilogue has most of the work, 24 warps of 80
+// (complex 8 x 32, 0.4 GiB of A: 577 -> 558 us with beta, 375 -> 341 without; 16 x 16: 527 with 16
+// warps, 653 with 24).
+constexpr int NSL = 8;
+__host__ __device__ constexpr int epi_groups(int nw) { return (nw - NSL) / 4; }
 constexpr int MAXAST = 3;                 // A' stages (at most)
-constexpr int CHUNK_BYTES = ROWS * 64;    // one chunk of old C: 8 doubles of each of 128 rows
+constexpr int CHUNK = 4;                  // output columns an epilogue warp converts at a time
+constexpr int CHUNK_BYTES = ROWS * CHUNK * 8;  // old C of one chunk
 constexpr uint32_t SLEEP_MMA = 32;        // ns between polls of the MMA thread
 // Per contraction width MP: the ring of row-exponent records (tiles), the header (barriers, TMEM
 // slot, column exponents, row exponents; a multiple of 1024), and the old-C chunks each epilogue
@@ -72,7 +72,7 @@ __host__ __device__ constexpr int row_ring() { return MP == 64 ? 4 : 8; }
 template <int MP>
 __host__ __device__ constexpr int hdr_bytes() { return MP == 64 ? 3072 : 5120; }
 template <int MP>
-__host__ __device__ constexpr int c_depth() { return MP == 64 ? 2 : (MP == 32 ? 3 : 4); }
+__host__ __device__ constexpr int c_depth() { return MP == 32 ? 6 : 4; }
 
 struct Args {
   const void* A;    // storage type T of the kernel (double or float), as B and C
@@ -103,18 +103,31 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo) {
   d |= (uint64_t)1 << 46;
   return d;
 }
-// issued by one elected lane of a converged warp, so that the operands stay warp-uniform
-__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p, e;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
-      " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+// One lane of a converged warp, the same one every time; it issues a whole block of MMAs and their
+// commit.  What an MMA costs the issuing warp is the instructions in front of it: with the election
+// and both descriptors put together for each MMA, 60 clocks on an idle SM and ~135 beside the
+// slicers; from bases and constant offsets, the tensor pipe's own 39 (N <= 64) to 64 (N = 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}\n" : "=r"(p));
+  return p != 0;
+}
+template <bool ACC>
+__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc) {
+  if constexpr (ACC)
+    asm volatile(
+        "{\n .reg .pred p;\n setp.eq.b32 p, 0, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            tmem),
+        "l"(da), "l"(db), "r"(idesc));
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, 0, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            tmem),
+        "l"(da), "l"(db), "r"(idesc));
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile(
-      "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
-      " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar))
-      : "memory");
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+               : "memory");
 }
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -323,10 +336,14 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int MP, typename T>
-__global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
-  constexpr int NSL = slicer_warps<MP>(), NEP = 16 - NSL, EG = epi_groups<MP>();
-  constexpr int TPS = NSL * 32 / ROWS;  // slicer threads per row (1 or 2)
+// HASC: old C is read (beta != 0 and not folded).  The two kinds of epilogue are compiled apart because
+// instruction fetch shows: with both in one kernel, 64 x 64 in place took 504 us at 512 MiB of A
+// instead of 434, 64 x 64 with beta 610 instead of 559.
+template <int MP, typename T, int NW, bool HASC>
+__global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
+  constexpr int THREADS = NW * 32;
+  constexpr int NEP = NW - NSL, EG = epi_groups(NW);
+  constexpr int TPS = NSL * 32 / ROWS;  // slicer threads per row (2 or 4)
   constexpr int PART = MP / TPS;        // A values per slicer thread
   constexpr int CD = c_depth<MP>();    // old-C chunks in flight per epilogue thread
   constexpr int RE = row_ring<MP>(), HDR = hdr_bytes<MP>();
@@ -350,9 +367,10 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
   // m in octets of 8 rows x 16 bytes (no swizzle); bytes between k-octets and between blocks:
   const uint32_t bko = 128u * (uint32_t)NB, bcb = (uint32_t)(MP / 8) * bko;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int64_t t_begin = p.ntiles * blockIdx.x / gridDim.x;
-  const int64_t t_end = p.ntiles * (blockIdx.x + 1) / gridDim.x;
-  const int nt = (int)(t_end - t_begin);
+  // tiles blockIdx.x, blockIdx.x + gridDim.x, ..: the CTAs read and write one window of the operands
+  // that moves along
+  const int nt = (int)((p.ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  const int64_t row0 = (int64_t)blockIdx.x * ROWS, rstep = (int64_t)gridDim.x * ROWS;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
@@ -408,31 +426,51 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
   // (after it has sliced its rows of the tile) or, where the epilogue has slack (no beta FMA, no
   // old C, few MMAs per tile) and the accumulator sets allow p.la >= 1 tiles of lookahead,
   // epilogue warp 8 (tile t + la before it drains tile t).
-  int mjob = 0;
-  auto issue_tile = [&](int it) -> bool {
-    const int s = it % p.nast;
-    if (!wait_ab(&afull[s], (uint32_t)((it / p.nast) & 1), abort_f, p.err, SLEEP_MMA)) return false;
+  const uint32_t idesc = (1u << 4) | ((uint32_t)((DIGITS * NB) >> 3) << 17) | ((128u >> 4) << 24);
+  const uint32_t istep = (uint32_t)(NB >> 3) << 17;  // one plane of B less
+  int ms = 0, mk = 0;          // next A' stage and accumulator set,
+  uint32_t mph = 0, kph = 0;   // and how often (mod 2) each ring has gone round
+  bool kwrap = false;          // every accumulator set has been used
+  auto issue_tile = [&]() -> bool {
+    const int s = ms;
+    if (!wait_ab(&afull[s], mph, abort_f, p.err, SLEEP_MMA)) return false;
     tc_after();
-    const uint32_t as = smem_u32(adig) + (uint32_t)s * p.astage;
-    for (int cb = 0; cb < p.ncb; cb++, mjob++) {
-      const int k = mjob % p.nsets;
-      if (mjob >= p.nsets) {
-        if (!wait_ab(&tempty[k], (uint32_t)((mjob / p.nsets - 1) & 1), abort_f, p.err, SLEEP_MMA)) return false;
+    const uint64_t da = make_desc(smem_u32(adig) + (uint32_t)s * p.astage, 2048u);
+    for (int cb = 0; cb < p.ncb; cb++) {
+      const int k = mk;
+      if (kwrap) {
+        if (!wait_ab(&tempty[k], kph ^ 1u, abort_f, p.err, SLEEP_MMA)) return false;
         tc_after();
       }
-      const uint32_t dcol = tmem + (uint32_t)(k * 8 * NB);
-      const uint32_t bb = smem_u32(bdig) + (uint32_t)cb * bcb;
+      if (++mk == p.nsets) {
+        mk = 0;
+        kph ^= 1u;
+        kwrap = true;
+      }
+      if (elect_one()) {
+        const uint32_t dcol = tmem + (uint32_t)(k * 8 * NB);
+        uint64_t db = make_desc(smem_u32(bdig) + (uint32_t)cb * bcb, bko);
 #pragma unroll
-      for (int ks = 0; ks < MP / 16; ks++)
+        for (int ks = 0; ks < MP / 16; ks++, db += bko >> 3) {
+          // digit 1 against all 8 planes covers every accumulator column: the first one overwrites
+          if (ks == 0)
+            mma_f16<false>(dcol, da, db, idesc);
+          else
+            mma_f16<true>(dcol, da + (uint64_t)(ks * 256), db, idesc);
 #pragma unroll
-        for (int i = 0; i < DIGITS; i++)
-          mma_f16(dcol + (uint32_t)(i * NB), make_desc(as + (uint32_t)(i * MP * 256 + ks * 4096), 2048u),
-                  make_desc(bb + (uint32_t)(2 * ks) * bko, bko),
-                  (1u << 4) | ((uint32_t)(((DIGITS - i) * NB) >> 3) << 17) | ((128u >> 4) << 24),
-                  (ks | i) ? 1u : 0u);
-      mma_commit(&tfull[k]);
+          for (int i = 1; i < DIGITS; i++)
+            mma_f16<true>(dcol + (uint32_t)(i * NB), da + (uint64_t)(i * MP * 16 + ks * 256), db,
+                          idesc - (uint32_t)i * istep);
+        }
+        mma_commit(&tfull[k]);
+        if (cb + 1 == p.ncb) mma_commit(&aempty[s]);
+      }
+      __syncwarp();
     }
-    mma_commit(&aempty[s]);
+    if (++ms == p.nast) {
+      ms = 0;
+      mph ^= 1u;
+    }
     return true;
   };
   if (warp < NSL) {
@@ -440,19 +478,21 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
     const int row = tid / TPS, part = tid % TPS, m0 = part * PART;
     double v[PART];
     auto load_tile = [&](int it) {
-      const int64_t r1 = (t_begin + it) * ROWS;
+      const int64_t r1 = row0 + it * rstep;
       load_row<PART, T>(p, r1, row, (int)((p.K - r1) < ROWS ? (p.K - r1) : ROWS), m0, v);
     };
     if (nt > 0) load_tile(0);
+    int s = 0, es = 0;
+    uint32_t sph = 1, eph = 1;  // parities of the releases waited for: the round before
     for (int it = 0; it < nt; it++) {
-      const int s = it % p.nast, es = it % RE;
       uint32_t emax = 0;
 #pragma unroll
       for (int j = 0; j < PART; j++) emax = max(emax, exp_field(v[j]));
-      if (TPS == 2) emax = max(emax, (uint32_t)__shfl_xor_sync(0xffffffffu, emax, 1));
+#pragma unroll
+      for (int o = 1; o < TPS; o *= 2) emax = max(emax, (uint32_t)__shfl_xor_sync(0xffffffffu, emax, o));
       bool ok = *abort_f == 0;
-      if (ok && it >= RE) ok = wait_ab(&eempty[es], (uint32_t)((it / RE - 1) & 1), abort_f, p.err);
-      if (ok && it >= p.nast) ok = wait_ab(&aempty[s], (uint32_t)((it / p.nast - 1) & 1), abort_f, p.err);
+      if (ok && it >= RE) ok = wait_ab(&eempty[es], eph, abort_f, p.err);
+      if (ok && it >= p.nast) ok = wait_ab(&aempty[s], sph, abort_f, p.err);
       if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp leaves together
       if (part == 0) erow[es * ROWS + row] = (int)emax;
       unsigned char* A_ = adig + (size_t)s * p.astage;
@@ -488,74 +528,88 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
       }
       if (it + 1 < nt) load_tile(it + 1);  // in flight while this tile's MMAs run
       // a wait that runs out sets the abort flag, which the slicers see at the next tile
-      if (warp == 0 && p.la == 0) issue_tile(it);
+      if (warp == 0 && (HASC || MP > 16 || p.la == 0)) issue_tile();
+      if (++es == RE) {
+        es = 0;
+        eph ^= 1u;
+      }
+      if (++s == p.nast) {
+        s = 0;
+        sph ^= 1u;
+      }
     }
-    if (warp == 0 && p.la == 0) {
-      mma_commit(mfin);  // completes once every MMA issued by the elected lanes has
+    if (warp == 0 && (HASC || MP > 16 || p.la == 0)) {
+      if (elect_one()) mma_commit(mfin);  // completes once every MMA issued by the elected lane has
+      __syncwarp();
       mbar_wait_bounded(mfin, 0, nullptr);
     }
     __syncwarp();
   } else {
     // ---- epilogue: warp NSL + 4 g + q of group g reads TMEM lanes 32q..32q+31 (rows of the tile)
     const int q = warp & 3, r = 32 * q + lane, eg = (warp - NSL) >> 2;
-    const int CH = (N + 7) >> 3;        // chunks of 8 output columns per row
+    const int CH = (N + CHUNK - 1) / CHUNK;  // chunks of output columns per row
     const int CHg = (CH - eg + EG - 1) / EG;  // chunks c = eg, eg + EG, .. of this warp per tile
-    const int cpb = NB >> 3;            // chunks per block (even)
-    const bool need_c = !p.beta_zero;
-    // the FP64-pipe finisher where the epilogue runs no beta FMA on that pipe (measured: with the
-    // FMA, the conversion makes the FP64 pipe the bottleneck even on one warp group)
-    const bool cvt = !need_c;
-    // old C prefetch cursor: this warp's next chunk (tile pf_it, chunk pf_c) goes to ring slot
-    // pf_g % CD; one commit group per chunk (empty past the last chunk)
-    int pf_it = 0, pf_c = eg, pf_g = 0;
+    const int cpb = NB / CHUNK;              // chunks per block
+    // old C prefetch cursor: this warp's next chunk (tile pf_it, chunk pf_c).  Ring: cp.async into slot
+    // pf_s, one commit group per chunk (empty past the last chunk), CD - 1 chunks ahead.  (One chunk
+    // ahead in registers instead: the load's latency shows, 64 x 64 610 -> 868 us.)
+    int pf_it = 0, pf_c = eg, pf_s = 0;
+    int64_t pf_row = row0 + r;
+    const T* pf_src = static_cast<const T*>(p.C) + pf_row * p.ldc;
+    auto advance = [&]() {
+      pf_c += EG;
+      if (pf_c >= CH) {
+        pf_c = eg;
+        pf_it++;
+        pf_row += rstep;
+        pf_src += rstep * p.ldc;
+      }
+    };
     auto issue = [&]() {
       if (pf_it < nt && CHg > 0) {
-        const int c = pf_c;
-        const int64_t rr = (t_begin + pf_it) * ROWS + r;
-        const bool live = rr < p.K;
-        const T* src = static_cast<const T*>(p.C) + rr * p.ldc + 8 * c;
-        unsigned char* dst = cbuf + (size_t)(eg * CD + pf_g % CD) * CHUNK_BYTES + r * 64;
+        const bool live = pf_row < p.K;
+        const T* src = pf_src + CHUNK * pf_c;
+        const int left = N - CHUNK * pf_c;
+        unsigned char* dst = cbuf + (uint32_t)(eg * CD + pf_s) * CHUNK_BYTES + r * (CHUNK * 8);
         constexpr int PER16 = 16 / (int)sizeof(T);  // elements per 16-byte piece
         if (p.vecc) {
 #pragma unroll
-          for (int x = 0; x < 8 / PER16; x++) {
-            const int left = N - (8 * c + PER16 * x);
-            const uint32_t bytes = live && left > 0 ? (uint32_t)(min(left, PER16) * (int)sizeof(T)) : 0u;
+          for (int x = 0; x < CHUNK / PER16; x++) {
+            const uint32_t bytes =
+                live && left > PER16 * x ? (uint32_t)(min(left - PER16 * x, PER16) * (int)sizeof(T)) : 0u;
             cp_async16(dst + 16 * x, bytes ? (const void*)(src + PER16 * x) : p.C, bytes);
           }
         } else {
 #pragma unroll
-          for (int x = 0; x < 8; x++) {
-            const uint32_t bytes = (live && 8 * c + x < N) ? (uint32_t)sizeof(T) : 0u;
+          for (int x = 0; x < CHUNK; x++) {
+            const uint32_t bytes = (live && left > x) ? (uint32_t)sizeof(T) : 0u;
             if constexpr (sizeof(T) == 8)
               cp_async8(dst + 8 * x, bytes ? (const void*)(src + x) : p.C, bytes);
             else
               cp_async4(dst + 4 * x, bytes ? (const void*)(src + x) : p.C, bytes);
           }
         }
-        pf_c += EG;
-        if (pf_c >= CH) {
-          pf_c = eg;
-          pf_it++;
-        }
+        advance();
       }
       cp_async_commit();
-      pf_g++;
+      if (++pf_s == CD) pf_s = 0;
     };
-    if (need_c)
+    T cold[4];  // old C of the chunk in hand
+    if constexpr (HASC) {
       for (int i = 0; i < CD - 1; i++) issue();
-    const bool issuer = p.la > 0 && warp == NSL;
+    }
+    const bool issuer = !HASC && MP == 16 && p.la > 0 && warp == NSL;
     if (issuer)
-      for (int j = 0; j < p.la && j < nt; j++) issue_tile(j);
-    int g = 0;  // this warp's chunks consumed so far
-    int job = 0;
+      for (int j = 0; j < p.la && j < nt; j++) issue_tile();
+    int gs = 0;  // ring slot of this warp's next chunk
+    int es = 0, k = 0;
+    uint32_t eph = 0, kp = 0;
     bool ok = true;
     for (int it = 0; it < nt && ok; it++) {
-      const int es = it % RE;
-      if (issuer && it + p.la < nt) issue_tile(it + p.la);  // a timeout sets the abort flag
-      const int64_t rr = (t_begin + it) * ROWS + r;
+      if (issuer && it + p.la < nt) issue_tile();  // a timeout sets the abort flag
+      const int64_t rr = row0 + it * rstep + r;
       const bool live = rr < p.K;
-      ok = wait_ab(&efull[es], (uint32_t)((it / RE) & 1), abort_f, p.err);
+      ok = wait_ab(&efull[es], eph, abort_f, p.err);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -563,10 +617,14 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
       const int e = erow[es * ROWS + r] - 1014;
       __syncwarp();
       if (lane == 0) mbar_arrive(&eempty[es]);
+      if (++es == RE) {
+        es = 0;
+        eph ^= 1u;
+      }
       T* crow = static_cast<T*>(p.C) + rr * p.ldc;
-      for (int cb = 0; cb < p.ncb; cb++, job++) {
-        const int k = job % p.nsets;
-        ok = wait_ab(&tfull[k], (uint32_t)((job / p.nsets) & 1), abort_f, p.err);
+      int c = eg;  // this warp's chunks are c = eg (mod EG)
+      for (int cb = 0; cb < p.ncb; cb++) {
+        ok = wait_ab(&tfull[k], kp, abort_f, p.err);
         if (!__all_sync(0xffffffffu, ok)) {
           ok = false;
           break;
@@ -574,29 +632,27 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
         tc_after();
         const uint32_t tb = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(k * 8 * NB);
         const int c_hi = min(CH, (cb + 1) * cpb);
-        // this warp's chunks of the block: c = eg (mod EG)
-        for (int c = cb * cpb + ((eg - cb * cpb) % EG + EG) % EG; c < c_hi; c += EG, g++) {
-          if (need_c) issue();  // chunk g + CD - 1, into the slot of chunk g - 1, read in full already
-          // the chunk in two halves of 4 columns: half the TMEM values live at a time, so that the
-          // conversion chains of a half fit the registers side by side
-          const unsigned char* cs = cbuf + (size_t)(eg * CD + g % CD) * CHUNK_BYTES + r * 64;
-          if (need_c) cp_async_wait<CD - 1>();  // this thread's copies of chunk g have landed
-#pragma unroll
-          for (int hh = 0; hh < 2; hh++) {
+        for (; c < c_hi; c += EG) {
+          const unsigned char* cs = cbuf + (uint32_t)(eg * CD + gs) * CHUNK_BYTES + r * (CHUNK * 8);
+          if constexpr (HASC) {
+            issue();  // into the slot of the last chunk, read in full already
+            if (++gs == CD) gs = 0;
+            cp_async_wait<CD - 1>();  // this thread's copies of the chunk have landed
+          }
+          {
             uint32_t raw[8][4];
 #pragma unroll
-            for (int L = 0; L < 8; L++) tmem_ld4(tb + (uint32_t)(L * NB + 8 * (c - cb * cpb) + 4 * hh), raw[L]);
-            double cold[4];
-            if (need_c) {
+            for (int L = 0; L < 8; L++) tmem_ld4(tb + (uint32_t)(L * NB + CHUNK * (c - cb * cpb)), raw[L]);
+            if constexpr (HASC) {
               if constexpr (sizeof(T) == 8) {
-                const double2 w0 = reinterpret_cast<const double2*>(cs)[2 * hh];
-                const double2 w1 = reinterpret_cast<const double2*>(cs)[2 * hh + 1];
+                const double2 w0 = reinterpret_cast<const double2*>(cs)[0];
+                const double2 w1 = reinterpret_cast<const double2*>(cs)[1];
                 cold[0] = w0.x;
                 cold[1] = w0.y;
                 cold[2] = w1.x;
                 cold[3] = w1.y;
               } else {
-                const float4 w = reinterpret_cast<const float4*>(cs)[hh];
+                const float4 w = reinterpret_cast<const float4*>(cs)[0];
                 cold[0] = w.x;
                 cold[1] = w.y;
                 cold[2] = w.z;
@@ -607,21 +663,20 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
             if (live) {
               // all four columns are formed (columns beyond N hold zero digits and exponent 0)
               // and masked only at the store
-              const int c0 = 8 * c + 4 * hh;
+              const int c0 = CHUNK * c;
               const int4 f = *reinterpret_cast<const int4*>(fcol + c0);
               const int fc[4] = {f.x, f.y, f.z, f.w};
               double out[4];
-              if (cvt) {
+              // the conversion runs on the FP64 pipe, next to the beta FMA: on all columns without
+              // beta, on half of them with it (16 x 16 with beta: 527 us with none, 503 with half)
 #pragma unroll
-                for (int x = 0; x < 4; x++) out[x] = window_cvt(level_window<MP>(raw, x), e + fc[x] - 1086);
-              } else {
-#pragma unroll
-                for (int x = 0; x < 4; x++) out[x] = window_int(level_window<MP>(raw, x), e + fc[x]);
-              }
-              if (need_c) {
+              for (int x = 0; x < 4; x++)
+                out[x] = !HASC || x < 2 ? window_cvt(level_window<MP>(raw, x), e + fc[x] - 1086)
+                                        : window_int(level_window<MP>(raw, x), e + fc[x]);
+              if constexpr (HASC) {
                 if (!p.cplx || p.beta[1] == 0.0) {  // a real beta scales both parts of a complex C alike
 #pragma unroll
-                  for (int x = 0; x < 4; x++) out[x] = fma(p.beta[0], cold[x], out[x]);
+                  for (int x = 0; x < 4; x++) out[x] = fma(p.beta[0], (double)cold[x], out[x]);
                 } else {
 #pragma unroll
                   for (int x = 0; x < 4; x += 2) {  // (re, im) pairs: c0 is a multiple of 4
@@ -649,11 +704,16 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmm_kernel(const Args p) {
         tc_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[k]);
+        if (++k == p.nsets) {
+          k = 0;
+          kp ^= 1u;
+        }
       }
     }
-    if (need_c) cp_async_wait<0>();
+    if constexpr (HASC) cp_async_wait<0>();
     if (issuer) {
-      mma_commit(mfin);
+      if (elect_one()) mma_commit(mfin);
+      __syncwarp();
       mbar_wait_bounded(mfin, 0, nullptr);
     }
   }
@@ -746,10 +806,11 @@ skinny_status split_tsmm_t(skinny_handle h, bool cplx, bool f32, int64_t M, int6
   a.astage = (uint32_t)(ROWS * DIGITS * MP * 2);
   a.bbytes = (uint32_t)round_up((int64_t)2 * DIGITS * MP * a.NM, 1024);
   const int HDR = MP == 64 ? hdr_bytes<64>() : (MP == 32 ? hdr_bytes<32>() : hdr_bytes<16>());
+  // contraction width 16, more than 16 columns out: 24 warps
+  const int nw = MP == 16 && a.NM > 16 ? 24 : 16;
   const int64_t cbytes =
-      (int64_t)(MP == 64 ? epi_groups<64>() * c_depth<64>()
-                         : (MP == 32 ? epi_groups<32>() * c_depth<32>() : epi_groups<16>() * c_depth<16>())) *
-      CHUNK_BYTES;
+      a.beta_zero ? 0 : (int64_t)epi_groups(nw) * (MP == 32 ? c_depth<32>() : c_depth<16>()) * CHUNK_BYTES;
+  static_assert(c_depth<16>() == c_depth<64>(), "ring depth");
   // the deepest A' ring that fits beside B' and the old-C rings (one stage at MP = 64)
   a.nast = 0;
   for (int ns = MAXAST; ns >= 1 && a.nast == 0; ns--)
@@ -767,22 +828,23 @@ skinny_status split_tsmm_t(skinny_handle h, bool cplx, bool f32, int64_t M, int6
   const int smem = (int)(HDR + (int64_t)a.bbytes + (int64_t)a.nast * a.astage + cbytes);
   int64_t grid = std::min<int64_t>((int64_t)h->dev.sms, a.ntiles);
   if (grid < 1) grid = 1;
-  static SmemAttr attr[6];
+  bool attr_ok = false;
   auto launch = [&](auto kern, SmemAttr& at) {
-    const bool ok = ensure_smem_attr(kern, smem, at);
-    if (ok) kern<<<(int)grid, THREADS, smem, st>>>(a);
-    return ok;
+    attr_ok = ensure_smem_attr(kern, smem, at);
+    if (attr_ok) kern<<<(int)grid, nw * 32, smem, st>>>(a);
   };
-  bool attr_ok;
-  if (!f32) {
-    attr_ok = MP == 16 ? launch(split_tsmm_kernel<16, double>, attr[0])
-              : MP == 32 ? launch(split_tsmm_kernel<32, double>, attr[1])
-                         : launch(split_tsmm_kernel<64, double>, attr[2]);
-  } else {
-    attr_ok = MP == 16 ? launch(split_tsmm_kernel<16, float>, attr[3])
-              : MP == 32 ? launch(split_tsmm_kernel<32, float>, attr[4])
-                         : launch(split_tsmm_kernel<64, float>, attr[5]);
+  static SmemAttr attr[16];
+#define SK_STSMM(X, W, I)                                                                   \
+  if (MP == X && nw == W) {                                                                 \
+    if (!f32)                                                                               \
+      a.beta_zero ? launch(split_tsmm_kernel<X, double, W, false>, attr[I])                 \
+                  : launch(split_tsmm_kernel<X, double, W, true>, attr[I + 1]);             \
+    else                                                                                    \
+      a.beta_zero ? launch(split_tsmm_kernel<X, float, W, false>, attr[I + 2])              \
+                  : launch(split_tsmm_kernel<X, float, W, true>, attr[I + 3]);              \
   }
+  SK_STSMM(16, 16, 0) SK_STSMM(16, 24, 4) SK_STSMM(32, 16, 8) SK_STSMM(64, 16, 12)
+#undef SK_STSMM
   if (!attr_ok) return SKINNY_DEVICE_ERROR;  // the error text is set
   count_launch();
   const cudaError_t e = cudaGetLastError();
