@@ -13,7 +13,7 @@
 //     balanced base-256 digits d_1..d_8 (d_1 in [-64, 64], the others in [-128, 127]).  The
 //     sign is applied to F before splitting, so the digits of a negative x are the digits of -F.
 //     When a column meets an element larger than 2^E allows, E is raised (with 4 bits of
-//     headroom) and a new epoch starts for the whole CTA.
+//     headroom) and a new epoch starts for the whole CTA (drained words do not mix exponents).
 //   * Digits are exact in FP16.  For a stage of 16 rows the digits are laid out as FP16 planes
 //     (K-major, no swizzle): A' holds 12 planes of 64 rows in the order
 //     [0, 1, 5 | 0, 2, 6 | 0, 3, 7 | 0, 4, 8] (0 = a zero plane, p = digit p of the 64 columns),
@@ -36,11 +36,20 @@
 //     of an epoch in registers.  FP64 arithmetic happens only when an epoch ends: the int64 words
 //     are converted, scaled by 2^(EA + EB - 2080) (levels 2..5) or 2^(EA + EB - 2112) (6..9) and
 //     added to the CTA's FP64 partials.
-//   * Warp roles: warps 0-7 slice (one column and 8 rows per thread; 4 rows in Gram mode, where
-//     B is A) and drain; warp 8 streams rows of A and B into a ring of FP64 stages with 1-D TMA
-//     bulk copies (one per row; 8-byte cp.async where rows are not 16-byte aligned); warp 9
-//     issues the MMAs.  Every wait is bounded; a wait that runs
+//   * Warp roles (28 warps): 0-15 slice (8 columns of A or B each, 4 rows per thread; Gram: 4 columns of
+//     A, 2 rows), 16-23 drain, 24 fetches rows of A and B into a ring of stages (1-D TMA bulk copies of
+//     dense rows; other rows by cp.async, warps 26 and 27 helping), 25 issues the MMAs and opens and
+//     closes the periods.  No two slicer warps wait for each other: a column's rows all lie with one
+//     warp, which raises its exponent by itself, leaves (stage, exponent before, since) for the drain
+//     warps and marks the stage for the MMA warp.  Every wait is bounded; a wait that runs
 //     out sets the error word and the CTA finishes without waiting further and writes no C.
+//   * Bound: a stage of 16 x (64 + 64) values takes ~1800 clocks, in which the schedulers issue in 67 %
+//     (slicing: ~28 instructions a value), the tensor pipe is busy in 900 (14 MMAs of 64) and a TMA
+//     copy of the same rows would take ~700.  With 8 warps that sliced and drained by turns and voted
+//     on the exponents of each stage it was 3600: each step of a stage (two mbarriers, the vote, the
+//     drain) was waited out by all of them.  Measured, K rows: f64 64 x 64, K = 2^20, 794 -> 431 us;
+//     32 x 32, K = 2^22, 1252 -> 745; 48 x 24, K = 2^20, 714 -> 358; Gram 64, K = 2^20, 738 -> 403;
+//     rows of 80 (64 x 64, K = 2^20) 776 -> 616; f32 64 x 64, K = 2^18, 308 -> 156.
 //   * Blocks of 64 x 64 (M or N > 64) run in the same launch, as do the row chunks of every
 //     block; the last CTA of a block (ticket) sums the chunks' partials in chunk order and
 //     applies alpha and beta.  Gram (A = B) computes the upper blocks only and mirrors them.
@@ -66,8 +75,12 @@ constexpr int PSTAGES = 8;   // stages per accumulation period (128 rows: exact 
 constexpr int DSLOTS = 3;    // digit slots
 constexpr int MAXR = 8;      // FP64 stages (at most)
 constexpr int HEAD = 4;      // exponent headroom granted when a column's exponent is raised
-constexpr int NSL = 256;     // slicer / drain threads (warps 0-7)
-constexpr int THREADS = NSL + 64;
+constexpr int SW = 16;       // slicer warps: 0-15
+constexpr int DW = 8;        // drain warps: 16-23
+constexpr int WPROD = SW + DW, WMMA = WPROD + 1;  // producer warps: WPROD and, for rows copied one by one, two more
+// seven warpgroups (the last one: producers and MMA issuer) launched with 72 registers a
+// thread, of which the slicers give back 8 and the last group 32 for the drain warps' 104
+constexpr int THREADS = 32 * (SW + DW + 4);
 constexpr int W = 64;        // block width
 constexpr uint32_t LBO_A = 12 * 64 * 16;  // bytes between the two k-octets of A'
 constexpr uint32_t LBO_B = 9 * 64 * 16;
@@ -87,7 +100,7 @@ struct Args {
   double alpha, beta;
   int beta_zero;
   int nblk, bm, sym;  // 64 x 64 blocks; sym: A == B, upper blocks only
-  int bulk;           // rows by bulk copy (16-byte aligned rows of even width)
+  int bulk;           // rows start and end on 16-byte boundaries
   int abase16, bbase16;  // A / B start on a 16-byte boundary (dense stages by one bulk copy)
   int rstages;
   uint32_t raw_stage;  // bytes per FP64 stage
@@ -107,6 +120,12 @@ __device__ __forceinline__ uint64_t desc(uint32_t saddr, uint32_t lbo) {
   d |= (uint64_t)(128 >> 4) << 32;              // 8-row-group stride
   d |= (uint64_t)1 << 46;
   return d;
+}
+// one lane of a converged warp, the same one every time
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -128,6 +147,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
@@ -138,24 +160,12 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// named barrier over the 256 slicer threads; returns 1 on every thread if pred holds on any
-__device__ __forceinline__ int slicers_any(int pred) {
-  int r;
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, 1, 256, p;\n selp.s32 %0, 1, 0, q;\n}\n"
-      : "=r"(r)
-      : "r"(pred)
-      : "memory");
-  return r;
-}
-__device__ __forceinline__ void slicers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-
 // bounded wait that also gives up as soon as another thread of the CTA has given up; the producer
 // and MMA warps sleep between polls so that their polling leaves issue slots to the slicers
 __device__ __forceinline__ bool wait_ab(uint64_t* bar, uint32_t parity, volatile int* ab, int* err,
@@ -170,6 +180,22 @@ __device__ __forceinline__ bool wait_ab(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
+// the same for the slicers, all lanes of a warp at once and without a branch where the phase is
+// complete already (a wait by one lane of a warp, with a warp barrier, cost ~150 clocks more); false: it ran out
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile int* ab) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b32 i, a;\n mov.b32 i, 0;\n"
+      "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n @p bra D_%=;\n"
+      " ld.volatile.shared.b32 a, [%3];\n add.u32 i, i, 1;\n"
+      " setp.lt.u32 q, i, 4194304;\n setp.eq.and.b32 q, a, 0, q;\n @q bra W_%=;\n"
+      "D_%=:\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<int*>(ab)))
+      : "memory");
+  return ok != 0;
+}
+
 // signed fixed-point value of x relative to exponent field E, offset for balanced base-256 digits
 __device__ __forceinline__ uint64_t fixed_g(double x, uint32_t E) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
@@ -180,6 +206,30 @@ __device__ __forceinline__ uint64_t fixed_g(double x, uint32_t E) {
   uint64_t F = sh < 64 ? ((mant << 9) >> sh) : 0ull;
   if (hi >> 31) F = 0ull - F;
   return F + 0x8080808080808080ull;
+}
+
+// the same for E > 64 (FP32: E > 64 above its exponents' offset), where zeros and subnormal numbers
+// shift out entirely and need no case of their own; sh = E - exponent field >= 0
+template <typename TI>
+__device__ __forceinline__ uint64_t fixed_fast(uint32_t hi, uint32_t lo, uint32_t sh) {
+  uint32_t H, L;
+  if constexpr (sizeof(TI) == 8) {
+    H = __funnelshift_l(lo, (hi & 0xFFFFFu) | 0x100000u, 9);
+    L = lo << 9;
+  } else {
+    H = ((hi & 0x7FFFFFu) | 0x800000u) << 6;
+    L = 0;
+  }
+  uint64_t F;
+  asm("shr.u64 %0, %1, %2;" : "=l"(F) : "l"(((uint64_t)H << 32) | L), "r"(sh));  // 0 from 64 on
+  const int64_t sg = (int32_t)hi >> 31;
+  return (F ^ (uint64_t)sg) - (uint64_t)sg + 0x8080808080808080ull;
+}
+// exponent field of x's magnitude (subnormal numbers: 1), 0 for zero; of the FP64 value for FP32
+__device__ __forceinline__ uint32_t exp_field(double x) {
+  const uint32_t mh = (uint32_t)__double2hiint(x) & 0x7FFFFFFFu;
+  const uint32_t e = mh >> 20;
+  return e == 0 && (mh | (uint32_t)__double2loint(x)) ? 1u : e;
 }
 
 // FP16 pair (digit of x, digit of y) from the word (byte_x, 0x64, byte_y, 0x64): value 1024 + g
@@ -197,7 +247,9 @@ __device__ __forceinline__ double pow2i(int e) {  // 2^e, clamped to the normal 
   return __hiloint2double((e + 1023) << 20, 0);
 }
 
-template <typename TI, bool FOLD>
+// GR: how Gram blocks occur (0: none, A and B differ; 1: the only block; 2: among others), so that the
+// two ways of slicing are compiled together only where a launch has both
+template <typename TI, bool FOLD, int GR>
 __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
   constexpr uint32_t ES = sizeof(TI);
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -205,13 +257,19 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
   uint64_t* raw_empty = raw_full + MAXR;                   // [MAXR]
   uint64_t* dfull = raw_full + 2 * MAXR;                   // [DSLOTS]
   uint64_t* dempty = dfull + 4;                            // [DSLOTS]
-  uint64_t* bar_fin = dempty + 4;
+  uint64_t* tfull = dempty + 4;                            // [2]: a TMEM set holds a finished period
+  uint64_t* tempty = tfull + 2;                            // [2]: and has been drained
+  uint64_t* bar_fin = tempty + 2;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 512);
   volatile int* abort_f = reinterpret_cast<volatile int*>(smem + 516);
-  volatile int* flags = reinterpret_cast<volatile int*>(smem + 528);  // [DSLOTS]
-  int* rec_epoch = reinterpret_cast<int*>(smem + 576);                // [2]
-  int* rec = reinterpret_cast<int*>(smem + 1024);                     // [2][128]: EA[64], EB[64]
-  int* acc_rec = reinterpret_cast<int*>(smem + 2048);                 // [128]
+  volatile int* nperiods = reinterpret_cast<volatile int*>(smem + 520);  // number of periods, once known
+  volatile int* vflag = reinterpret_cast<volatile int*>(smem + 544);  // [4]: stage + 1 where an exponent is raised
+  volatile int* mstart = reinterpret_cast<volatile int*>(smem + 576);  // [2]: first stage of a TMEM set's period,
+  volatile int* mend = mstart + 2;                                     // [2]: the stage after its last,
+  volatile int* mepoch = mstart + 4;                                   // [2]: its epoch
+  volatile int* dprog = reinterpret_cast<volatile int*>(smem + 640);  // [DW]: periods up to here have their exponents
+  // [128] exponents of A's and B's columns: (stage of the last raise, before, since)
+  volatile uint64_t* rec = reinterpret_cast<volatile uint64_t*>(smem + 1024);
   unsigned char* dig = smem + HDR;
   unsigned char* raw = dig + DSLOTS * SLOT;
 
@@ -234,7 +292,7 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
   const TI* Ab = static_cast<const TI*>(p.A) + W * bi;
   const TI* Bb = static_cast<const TI*>(p.sym ? p.A : p.B) + W * bj;
   const int64_t ldb = p.sym ? p.lda : p.ldb;
-  const bool gram = p.sym && bi == bj;
+  const bool gram = GR == 0 ? false : GR == 1 ? true : p.sym && bi == bj;
   const int64_t s_begin = p.nstages * chunk / nchunks, s_end = p.nstages * (chunk + 1) / nchunks;
   const int nst = (int)(s_end - s_begin);
   const int R = p.rstages;
@@ -246,21 +304,34 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
   const int SR = FOLD ? 2 * ROWS : ROWS, rw = FOLD ? W / 2 : W;
   const int rsa = dense_a ? Mb : rw, rsb = dense_b ? Nb : rw;
 
+  const bool allbulk = p.bulk && dense_a && (gram || dense_b);  // one bulk copy per operand and stage
+
+  // slicer warps with a column: 8 columns of A or B each (Gram: 4 of A)
+  const int nslice = (FOLD ? 2 : 1) * (gram ? (Mb + 3) / 4 : (Mb + 7) / 8 + (Nb + 7) / 8);
+
+  if (tid < 128) rec[tid] = 0;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tslot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
     for (int s = 0; s < R; s++) {
-      mbar_init(&raw_full[s], p.bulk ? 1 : 32);
-      mbar_init(&raw_empty[s], 8);
+      mbar_init(&raw_full[s], allbulk ? 1 : 96);
+      mbar_init(&raw_empty[s], nslice);
     }
     for (int s = 0; s < DSLOTS; s++) {
-      mbar_init(&dfull[s], 8);
+      mbar_init(&dfull[s], nslice);
       mbar_init(&dempty[s], 1);
     }
+    for (int s = 0; s < 2; s++) {
+      mbar_init(&tfull[s], 2);
+      mbar_init(&tempty[s], DW);
+    }
+    for (int s = 0; s < 4; s++) vflag[s] = 0;
+    for (int s = 0; s < DW; s++) dprog[s] = 0;
     mbar_init(bar_fin, 1);
     *abort_f = 0;
+    *nperiods = 0x7fffffff;
     fence_mbar_init();
   }
   // zero planes and unused columns stay zero: clear every digit slot once
@@ -272,344 +343,413 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
   tc_after();
   const uint32_t tmem = *tslot;
 
-  if (warp == 8) {
-    // ---- producer: FP64 rows of A and B into the stage ring -------------------------------------
-    int issued = 0;
-    for (int ls = 0; ls < nst; ls++) {
-      const int rs = ls % R, use = ls / R;
-      if (use > 0) {
-        int ok = 0;
-        if (lane == 0) ok = wait_ab(&raw_empty[rs], (uint32_t)((use - 1) & 1), abort_f, p.err, 64);
-        if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      }
-      const int64_t row0 = (s_begin + ls) * SR;
-      const int rows = (int)min((int64_t)SR, p.K - row0);
-      TI* dA = reinterpret_cast<TI*>(raw + (size_t)rs * p.raw_stage);
-      TI* dB = dA + ROWS * W;
-      if (p.bulk) {
-        if (lane == 0) mbar_arrive_expect_tx(&raw_full[rs], (uint32_t)(rows * (Mb + (gram ? 0 : Nb)) * ES));
-        __syncwarp();
-        // dense rows (ld == block width): the stage is one contiguous copy; otherwise one per row
-        if (dense_a && lane == 0) bulk_g2s(dA, Ab + row0 * p.lda, (uint32_t)(rows * Mb * ES), &raw_full[rs]);
-        if (!gram && dense_b && lane == 1) bulk_g2s(dB, Bb + row0 * ldb, (uint32_t)(rows * Nb * ES), &raw_full[rs]);
-        const int na = dense_a ? 0 : rows, nb = (gram || dense_b) ? 0 : rows;
-        for (int r = lane; r < na + nb; r += 32) {
-          if (r < na)
-            bulk_g2s(dA + r * rw, Ab + (row0 + r) * p.lda, (uint32_t)(Mb * ES), &raw_full[rs]);
-          else
-            bulk_g2s(dB + (r - na) * rw, Bb + (row0 + r - na) * ldb, (uint32_t)(Nb * ES), &raw_full[rs]);
-        }
-      } else {
-        // rows not all 16-byte aligned (odd widths or leading dimensions): a dense operand whose
-        // stage starts and ends on 16-byte boundaries (always but for an odd last stage) is one
-        // bulk copy, announced on the barrier without an arrival; the rest element by element;
-        // one arrival per lane once its element copies have landed
-        const bool sa = dense_a && (row0 * Mb * ES) % 16 == 0 && (rows * Mb * ES) % 16 == 0;
-        const bool sb = !gram && dense_b && (row0 * Nb * ES) % 16 == 0 && (rows * Nb * ES) % 16 == 0;
-        if (lane == 0 && (sa || sb)) {
-          mbar_expect_tx(&raw_full[rs], (uint32_t)(((sa ? rows * Mb : 0) + (sb ? rows * Nb : 0)) * ES));
-          if (sa) bulk_g2s(dA, Ab + row0 * p.lda, (uint32_t)(rows * Mb * ES), &raw_full[rs]);
-          if (sb) bulk_g2s(dB, Bb + row0 * ldb, (uint32_t)(rows * Nb * ES), &raw_full[rs]);
-        }
-        if (!sa)
-          for (int e = lane; e < rows * Mb; e += 32) {
-            const int r = e / Mb, c = e - r * Mb;
-            if constexpr (ES == 8)
-              cp_async8(dA + r * rsa + c, Ab + (row0 + r) * p.lda + c);
-            else
-              cp_async4(dA + r * rsa + c, Ab + (row0 + r) * p.lda + c);
-          }
-        if (!gram && !sb)
-          for (int e = lane; e < rows * Nb; e += 32) {
-            const int r = e / Nb, c = e - r * Nb;
-            if constexpr (ES == 8)
-              cp_async8(dB + r * rsb + c, Bb + (row0 + r) * ldb + c);
-            else
-              cp_async4(dB + r * rsb + c, Bb + (row0 + r) * ldb + c);
-          }
-        cp_async_arrive(&raw_full[rs]);
-      }
-      issued = ls + 1;
-    }
-    // copies in flight must land before the CTA ends
-    if (!p.bulk) asm volatile("cp.async.wait_all;" ::: "memory");
-    if (lane == 0)
-      for (int ls = max(0, issued - R); ls < issued; ls++)
-        mbar_wait_bounded(&raw_full[ls % R], (uint32_t)((ls / R) & 1), nullptr);
-  } else if (warp == 9) {
-    // ---- MMA issuer ------------------------------------------------------------------------------
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);  // F32 <- F16 x F16
-      const uint32_t dig0 = smem_u32(dig);
-      int issued = 0;
+  if (warp >= WPROD) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    const int pw = warp == WPROD ? 0 : warp - WMMA;  // of 3 producer warps
+    if (warp != WMMA && (pw == 0 || !allbulk)) {
+      // ---- producer: FP64 rows of A and B into the stage ring -------------------------------------
+      int issued = 0, rs = -1;
+      uint32_t rph = 1;  // parity of the releases waited for: the round before
       for (int ls = 0; ls < nst; ls++) {
-        const int ds = ls % DSLOTS;
-        if (!wait_ab(&dfull[ds], (uint32_t)((ls / DSLOTS) & 1), abort_f, p.err, 32)) break;
+        if (++rs == R) {
+          rs = 0;
+          rph ^= 1u;
+        }
+        if (ls >= R) {
+          int ok = 0;
+          if (lane == 0) ok = wait_ab(&raw_empty[rs], rph, abort_f, p.err, 64);
+          if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        }
+        const int64_t row0 = (s_begin + ls) * SR;
+        const int rows = (int)min((int64_t)SR, p.K - row0);
+        TI* dA = reinterpret_cast<TI*>(raw + (size_t)rs * p.raw_stage);
+        TI* dB = dA + ROWS * W;
+        if (allbulk) {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&raw_full[rs], (uint32_t)(rows * (Mb + (gram ? 0 : Nb)) * ES));
+            bulk_g2s(dA, Ab + row0 * p.lda, (uint32_t)(rows * Mb * ES), &raw_full[rs]);
+            if (!gram) bulk_g2s(dB, Bb + row0 * ldb, (uint32_t)(rows * Nb * ES), &raw_full[rs]);
+          }
+        } else {
+          // a dense operand whose stage starts and ends on 16-byte boundaries (always but for an odd
+          // last stage) is one bulk copy, announced on the barrier without an arrival; other rows are
+          // copied by all lanes, 16 bytes each where the rows are aligned (a bulk copy per row costs
+          // ~100 clocks: 3600 a stage of 32 rows), else element by element; one arrival per lane once
+          // its copies have landed
+          const bool sa = dense_a && (row0 * Mb * ES) % 16 == 0 && (rows * Mb * ES) % 16 == 0;
+          const bool sb = !gram && dense_b && (row0 * Nb * ES) % 16 == 0 && (rows * Nb * ES) % 16 == 0;
+          if (pw == 0 && lane == 0 && (sa || sb)) {
+            mbar_expect_tx(&raw_full[rs], (uint32_t)(((sa ? rows * Mb : 0) + (sb ? rows * Nb : 0)) * ES));
+            if (sa) bulk_g2s(dA, Ab + row0 * p.lda, (uint32_t)(rows * Mb * ES), &raw_full[rs]);
+            if (sb) bulk_g2s(dB, Bb + row0 * ldb, (uint32_t)(rows * Nb * ES), &raw_full[rs]);
+          }
+          if (p.bulk) {
+            const int ca = Mb * ES / 16, cb = Nb * ES / 16;  // <= 32
+            if (!sa && lane < ca)
+              for (int r = pw; r < rows; r += 3)
+                cp_async16(dA + r * rsa + lane * (16 / ES), Ab + (row0 + r) * p.lda + lane * (16 / ES));
+            if (!gram && !sb && lane < cb)
+              for (int r = pw; r < rows; r += 3)
+                cp_async16(dB + r * rsb + lane * (16 / ES), Bb + (row0 + r) * ldb + lane * (16 / ES));
+          }
+          if (!sa && !p.bulk)
+            for (int e = 32 * pw + lane; e < rows * Mb; e += 96) {
+              const int r = e / Mb, c = e - r * Mb;
+              if constexpr (ES == 8)
+                cp_async8(dA + r * rsa + c, Ab + (row0 + r) * p.lda + c);
+              else
+                cp_async4(dA + r * rsa + c, Ab + (row0 + r) * p.lda + c);
+            }
+          if (!gram && !sb && !p.bulk)
+            for (int e = 32 * pw + lane; e < rows * Nb; e += 96) {
+              const int r = e / Nb, c = e - r * Nb;
+              if constexpr (ES == 8)
+                cp_async8(dB + r * rsb + c, Bb + (row0 + r) * ldb + c);
+              else
+                cp_async4(dB + r * rsb + c, Bb + (row0 + r) * ldb + c);
+            }
+          cp_async_arrive(&raw_full[rs]);
+        }
+        issued = ls + 1;
+      }
+      // copies in flight must land before the CTA ends
+      if (!allbulk) asm volatile("cp.async.wait_all;" ::: "memory");
+      if (lane == 0)
+        for (int ls = max(0, issued - R); ls < issued; ls++)
+          mbar_wait_bounded(&raw_full[ls % R], (uint32_t)((ls / R) & 1), nullptr);
+    } else if (warp == WMMA) {
+      // ---- MMA issuer: one elected lane, descriptors from a base and constant offsets; opens and closes
+      // the periods ---------------------------------------------------------------------------------------
+      const uint32_t idesc = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);  // F32 <- F16 x F16
+      int ds = 0, periods = 0, ls = 0, pstart = 0, epoch = 0, epoch_periods = 0;
+      uint32_t dph = 0;
+      for (; ls < nst; ls++) {
+        if (!__all_sync(0xffffffffu, wait_ab(&dfull[ds], dph, abort_f, p.err, 32))) break;
+        const bool raised = vflag[ls & 3] == ls + 1;
+        const bool start = ls == 0 || raised || ls - pstart >= PSTAGES || epoch_periods >= MAX_EPOCH_PERIODS;
+        if (start) {
+          if (raised || ls == 0 || epoch_periods >= MAX_EPOCH_PERIODS) {
+            epoch++;
+            epoch_periods = 0;
+          }
+          epoch_periods++;
+          pstart = ls;
+          const int buf = periods & 1;
+          if (periods >= 2 &&
+              !__all_sync(0xffffffffu, wait_ab(&tempty[buf], (uint32_t)(((periods >> 1) - 1) & 1), abort_f, p.err)))
+            break;
+          if (elect_one()) {
+            if (periods) {  // the period before is complete
+              mend[buf ^ 1] = ls;
+              mma_commit(&tfull[buf ^ 1]);
+              mbar_arrive(&tfull[buf ^ 1]);
+            }
+            mstart[buf] = ls;
+            mepoch[buf] = epoch;
+          }
+          __syncwarp();
+          periods++;
+        }
         tc_after();
-        const int f = flags[ds];
-        const uint32_t start = f & 1, buf = (f >> 1) & 1;
-        const uint32_t a0 = dig0 + ds * SLOT, b0 = a0 + SLOT_A;
-        const uint32_t d0 = tmem + buf * 256;
-#pragma unroll
-        for (int i = -3; i <= 2; i++)
-          mma_f16(d0, desc(a0 + slot_a(i) * 1024, LBO_A), desc(b0 + (2 - i) * 1024, LBO_B), idesc,
-                  (start && i == -3) ? 0u : 1u);
-#pragma unroll
-        for (int i = -3; i <= 4; i++)
-          mma_f16(d0 + 128, desc(a0 + slot_a(i) * 1024, LBO_A), desc(b0 + (4 - i) * 1024, LBO_B), idesc,
-                  (start && i == -3) ? 0u : 1u);
-        mma_commit(&dempty[ds]);
-        issued++;
+        const uint32_t a0 = smem_u32(dig) + ds * SLOT;
+        if (elect_one()) {
+          const uint64_t da = desc(a0, LBO_A), db = desc(a0 + SLOT_A, LBO_B);  // planes are 1024 bytes apart
+          const uint32_t d0 = tmem + ((periods - 1) & 1) * 256;
+  #pragma unroll
+          for (int i = -3; i <= 2; i++)
+            mma_f16(d0, da + 64 * slot_a(i), db + 64 * (2 - i), idesc, i == -3 ? !start : 1u);
+  #pragma unroll
+          for (int i = -3; i <= 4; i++)
+            mma_f16(d0 + 128, da + 64 * slot_a(i), db + 64 * (4 - i), idesc, i == -3 ? !start : 1u);
+          mma_commit(&dempty[ds]);
+        }
+        __syncwarp();
+        if (++ds == DSLOTS) {
+          ds = 0;
+          dph ^= 1u;
+        }
       }
-      if (issued) {  // every MMA has finished before the TMEM is released
-        mma_commit(bar_fin);
-        mbar_wait_bounded(bar_fin, 0, nullptr);
+      // (the set that the closing arrival is made on must have been drained: a drain warp that had not
+      // yet seen its last period would otherwise wait for a phase that is past)
+      if (periods >= 2) wait_ab(&tempty[periods & 1], (uint32_t)(((periods >> 1) - 1) & 1), abort_f, p.err);
+      __syncwarp();
+      if (elect_one()) {
+        const int buf = periods & 1;
+        if (periods) {
+          mend[buf ^ 1] = ls;
+          mma_commit(&tfull[buf ^ 1]);
+          mbar_arrive(&tfull[buf ^ 1]);
+          mma_commit(bar_fin);
+        }
+        *nperiods = periods;
+        mbar_arrive(&tfull[buf]);
+        mbar_arrive(&tfull[buf]);
       }
+      __syncwarp();
+      if (periods) mbar_wait_bounded(bar_fin, 0, nullptr);  // every MMA has finished before the TMEM is released
     }
-  } else {
-    // ---- slicers / drain (warps 0-7) ------------------------------------------------------------
-    // slicing unit: column c of A or B and 8 rows (Gram: column c of A and 4 rows).  Lanes are
-    // laid out so that a half-warp reads 16 consecutive columns of one row (no bank conflicts)
-    // and a quarter-warp stores 128 contiguous bytes of digits.
-    const bool isB = !gram && warp >= 4;
-    const int c = gram ? 8 * warp + (lane & 7) : 16 * (warp & 3) + (lane & 15);
-    const int sub = gram ? (lane >> 3) : (lane >> 4);
-    const int nrow = gram ? 4 : 8;
-    // folded stages: plane row c holds column c % 32 of the stage's row half c / 32
-    const int cact = FOLD ? (c & 31) : c, rbase = FOLD ? ROWS * (c >> 5) : 0;
-    const bool cvalid = cact < (isB ? Nb : Mb);
-    const int cofs = (c >> 3) * 128 + (c & 7) * 16;  // row c of a digit plane (8-row core groups)
-    uint32_t Ecur = 0;
-    // drain cells: TMEM lane 32 q + lane (q = warp % 4), C column block [32 nh, 32 nh + 32)
-    const int q = warp & 3, nh = warp >> 2;
+  } else if (warp >= SW) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    // ---- drain: TMEM -> one int64 word per cell and lane half; FP64 where an epoch ends ---------------
+    // cells: TMEM lane 32 q + lane (q = warp % 4), C columns [32 nh, 32 nh + 32)
+    const int q = warp & 3, nh = (warp >> 2) & 1;
     const int hm = q >> 1;                  // 0: levels 2..5, 1: levels 6..9
     const int m = (32 * q + lane) & 63;
-    // cells this thread keeps: folded stages keep the two diagonal quadrants only
+    // cells this warp keeps: folded stages keep the two diagonal quadrants only
     const bool live = !FOLD || (q & 1) == nh;
-    const int mv = FOLD ? (m & 31) : m, nofs = FOLD ? 32 * nh : 0;
+    const int mv = FOLD ? (m & 31) : m, nlim = min(32, Nb - (FOLD ? 0 : 32 * nh));
     long long acc[32];
 #pragma unroll
     for (int x = 0; x < 32; x++) acc[x] = 0;
-    int acc_epoch = -1;
+    int acc_epoch = -1, ea = 0, eb = 0;  // exponents of row m; of column 32 nh + lane
     bool flushed = false;
-    double* part = p.partials + ((size_t)(blk * nchunks + chunk) * 2 + hm) * 4096;
-
-    auto flush = [&]() {
-      const int ea = acc_rec[m];
+    double* part = p.partials + ((size_t)(blk * nchunks + chunk) * 2 + hm) * 4096 + (32 * nh) * 64 + m;
+    for (int idx = 0;; idx++) {
+      const int buf = idx & 1;
+      int ok = 1;
+      if (lane == 0) ok = wait_ab(&tfull[buf], (uint32_t)((idx >> 1) & 1), abort_f, p.err, 300);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      const bool last = !ok || *nperiods == idx;
+      const int ep = last ? -2 : mepoch[buf];
+      if (ep != acc_epoch) {  // warp-uniform: the words so far are complete
+        // (one multiplication where the power of two is in range: the FP64 pipe does 1.89 a clock)
+        if (live && (acc_epoch >= 0 || last)) {
 #pragma unroll
-      for (int x = 0; x < 32; x++) {
-        const int n = 32 * nh + x;
-        if (live && mv < Mb && n - nofs < Nb) {
-          double v = 0.0;
-          if (acc_epoch >= 0)
-            v = (double)acc[x] * pow2i(ea - 1040) * pow2i(acc_rec[64 + n] - 1040 - (hm ? 32 : 0));
-          double* d = part + n * 64 + m;
-          *d = flushed ? *d + v : v;
+          for (int x = 0; x < 32; x++) {
+            const int ebx = __shfl_sync(0xffffffffu, eb, x) - 1040 - (hm ? 32 : 0), es = ea - 1040 + ebx;
+            if (mv < Mb && x < nlim) {
+              double v = (double)acc[x];
+              v = (unsigned)(es + 1022) <= 2045u ? v * pow2i(es) : v * pow2i(ea - 1040) * pow2i(ebx);
+              part[x * 64] = flushed ? part[x * 64] + v : v;
+            }
+            acc[x] = 0;
+          }
+          flushed = true;
         }
-        acc[x] = 0;
+        if (last) break;
+        acc_epoch = ep;
+        const uint32_t first = (uint32_t)mstart[buf];
+        auto exponent = [&](int i) {
+          const uint64_t r = rec[i];
+          return (int)(first >= (uint32_t)(r >> 32) ? r & 0xFFFFu : (r >> 16) & 0xFFFFu);
+        };
+        ea = exponent(m);
+        eb = exponent((gram ? 0 : 64) + 32 * nh + lane);
       }
-      flushed = true;
-    };
-    // drain piece k (cells 8k..8k+7 of this thread) of the TMEM set `buf`; piece 0 first closes
-    // the accumulators' epoch when the period belongs to a new one
-    auto drain_piece = [&](int buf, int k) {
-      if (k == 0) {
-        const int ep = rec_epoch[buf];
-        if (ep != acc_epoch) {  // uniform: a new epoch begins with this period
-          flush();
-          slicers_sync();
-          if (tid < 128) acc_rec[tid] = rec[buf * 128 + tid];
-          slicers_sync();
-          acc_epoch = ep;
-        }
-      }
+      __syncwarp();
+      if (lane == 0) dprog[warp - SW] = mend[buf];
       tc_after();
       const uint32_t tb = tmem + ((uint32_t)(32 * q) << 16) + buf * 256 + 32 * nh;
+      if (live) {
 #pragma unroll
-      for (int hp = 0; hp < 4; hp++) {
-        if (hp != k || !live) continue;
-        uint32_t s0[8], s1[8], s2[8], s3[8];
-        tmem_ld8(tb + hp * 8, s0);          // key 2, columns j   : level 2 / 6
-        tmem_ld8(tb + 64 + hp * 8, s1);     // key 2, columns j+1 : level 3 / 7
-        tmem_ld8(tb + 128 + hp * 8, s2);    // key 4, columns j   : level 4 / 8
-        tmem_ld8(tb + 192 + hp * 8, s3);    // key 4, columns j+1 : level 5 / 9
-        tmem_wait_ld();
+        for (int hp = 0; hp < 8; hp++) {
+          uint32_t s0[4], s1[4], s2[4], s3[4];
+          tmem_ld4(tb + hp * 4, s0);          // key 2, columns j   : level 2 / 6
+          tmem_ld4(tb + 64 + hp * 4, s1);     // key 2, columns j+1 : level 3 / 7
+          tmem_ld4(tb + 128 + hp * 4, s2);    // key 4, columns j   : level 4 / 8
+          tmem_ld4(tb + 192 + hp * 4, s3);    // key 4, columns j+1 : level 5 / 9
+          tmem_wait_ld();
 #pragma unroll
-        for (int x = 0; x < 8; x++) {
-          const long long l0 = __float2int_rn(__uint_as_float(s0[x]));
-          const long long l1 = __float2int_rn(__uint_as_float(s1[x]));
-          const long long l2 = __float2int_rn(__uint_as_float(s2[x]));
-          const long long l3 = __float2int_rn(__uint_as_float(s3[x]));
-          acc[hp * 8 + x] += (l0 << 24) + (l1 << 16) + (l2 << 8) + l3;
+          for (int x = 0; x < 4; x++) {
+            long long a = acc[hp * 4 + x] + __float2int_rn(__uint_as_float(s3[x]));
+            a += (long long)__float2int_rn(__uint_as_float(s2[x])) * (1 << 8);
+            a += (long long)__float2int_rn(__uint_as_float(s1[x])) * (1 << 16);
+            a += (long long)__float2int_rn(__uint_as_float(s0[x])) * (1 << 24);
+            acc[hp * 4 + x] = a;
+          }
         }
       }
       tc_before();
-    };
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[buf]);
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // ---- slicers --------------------------------------------------------------------------------------
+    // slicing unit: column c of A or B and 4 rows (Gram: column c of A and 2 rows).  All 16 rows of a
+    // column lie with one warp, so that its exponent is this warp's own affair: a warp that raises
+    // one marks the stage, and the MMA warp begins a new period there.
+    const bool isB = !gram && warp >= SW / 2;
+    const int c = gram ? 4 * warp + (lane & 3) : 8 * (warp & 7) + (lane & 7);
+    const int sub = gram ? lane >> 2 : lane >> 3;
+    constexpr int NR = GR == 1 ? 2 : 4;  // rows read (Gram among other blocks: 2 of them count)
+    const int nrow = gram ? 2 : 4;
+    // folded stages: plane row c holds column c % 32 of the stage's row half c / 32
+    const int cact = FOLD ? (c & 31) : c, r0 = (FOLD ? ROWS * (c >> 5) : 0) + sub * nrow;
+    const bool cvalid = cact < (isB ? Nb : Mb);
+    const int cofs = (c >> 3) * 128 + (c & 7) * 16;  // row c of a digit plane (8-row core groups)
+    // the column's exponent; unused columns read column 0 and never raise theirs
+    uint32_t Ecur = cvalid ? 0u : 4000u;
+    // FP64 exponent fields = own fields + EOFS; columns up to EMIN (zeros, subnormal numbers in
+    // range) are sliced by the general code
+    constexpr bool F32 = ES == 4;
+    constexpr uint32_t EOFS = F32 ? 896 : 0, EMIN = EOFS + 64;
+    // (FP32 columns that reach 2^124 too: infinities keep the exponent field of their FP64 value)
+    bool slow = true;  // warp-uniform: a column of this warp is such a one
+    const int rstr = isB ? rsb : rsa;
+    const int tofs = (isB ? ROWS * W : 0) + r0 * rstr + (cvalid ? cact : 0);
 
-    int cur_buf = 1, pstart = 0, epoch = 0, epoch_periods = 0;
-    // the period before the current one is drained in 4 pieces over the stages that follow the
-    // completion of its last MMAs, so that the conversions interleave with slicing
-    int pend = 0, pend_buf = 0, pend_last = 0, pend_piece = 0;
-    for (int ls = 0; ls < nst; ls++) {
-      const int rs = ls % R, ds = ls % DSLOTS;
-      const int64_t row0 = (s_begin + ls) * SR;
-      const int rows = (int)min((int64_t)SR, p.K - row0);
-      // lane 0 waits for the FP64 stage (TMA) and for the MMAs that read the digit slot; the
-      // warp barrier then orders the other lanes' reads and writes after those waits
-      if (lane == 0) {
-        wait_ab(&raw_full[rs], (uint32_t)((ls / R) & 1), abort_f, p.err);
-        if (ls >= DSLOTS) wait_ab(&dempty[ds], (uint32_t)(((ls / DSLOTS) - 1) & 1), abort_f, p.err);
-      }
-      __syncwarp();
-      // load my unit and its column maximum
-      const TI* T = reinterpret_cast<const TI*>(raw + (size_t)rs * p.raw_stage) + (isB ? ROWS * W : 0);
-      const int rstr = isB ? rsb : rsa;
-      // column maximum of |x| from the high words (the exponent field of the largest high word is
-      // the largest exponent field); nonzero low words mark subnormals in an otherwise zero column
-      double v[8];
-      uint32_t mh = 0, ol = 0;
+    struct Unit {
+      uint32_t hi[NR], lo[NR];  // the elements' bits (FP32: hi)
+    };
+    auto value = [](const Unit& u, int k) {
+      return F32 ? (double)__uint_as_float(u.hi[k]) : __hiloint2double((int)u.hi[k], (int)u.lo[k]);
+    };
+    auto field = [](const Unit& u, int k) { return F32 ? (u.hi[k] >> 23) & 0xFFu : (u.hi[k] >> 20) & 0x7FFu; };
+    int rs = -1, ds = -1, ok = 1, raised = 0;  // ok: every wait has ended in time; raised: stage of the last raise
+    uint32_t rph = 1, dph = 1;
+    const bool wvalid = __any_sync(0xffffffffu, cvalid);  // (a warp without a column has nothing to do)
+    for (int ls = 0; wvalid && ls < nst; ls++) {
+      Unit cur;
+      if (++rs == R) rs = 0;
+      if (rs == 0) rph ^= 1u;
+      if (++ds == DSLOTS) ds = 0;
+      if (ds == 0) dph ^= 1u;
+      ok &= wait_warp(&raw_full[rs], rph, abort_f);
+      const int rows = (int)min((int64_t)SR, p.K - (s_begin + ls) * SR);
+      const TI* T = reinterpret_cast<const TI*>(raw + (size_t)rs * p.raw_stage) + tofs;
+      auto get = [&](int k) {
+        if constexpr (F32) {
+          cur.hi[k] = __float_as_uint(T[k * rstr]);
+        } else {
+          const double x = T[k * rstr];
+          cur.hi[k] = (uint32_t)__double2hiint(x);
+          cur.lo[k] = (uint32_t)__double2loint(x);
+        }
+      };
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int rr = rbase + sub * nrow + k;
-        v[k] = (k < nrow && cvalid && rr < rows) ? (double)T[rr * rstr + cact] : 0.0;
-        mh = max(mh, (uint32_t)__double2hiint(v[k]) & 0x7FFFFFFFu);
-        ol |= (uint32_t)__double2loint(v[k]);
+      for (int k = 0; k < NR; k++) cur.hi[k] = cur.lo[k] = 0;
+      if (rows == SR) {
+#pragma unroll
+        for (int k = 0; k < NR; k++)
+          if (GR < 2 || k < nrow) get(k);
+      } else {
+#pragma unroll
+        for (int k = 0; k < NR; k++)
+          if ((GR < 2 || k < nrow) && r0 + k < rows) get(k);
       }
-      if (gram) {
-        mh = max(mh, __shfl_xor_sync(0xffffffffu, mh, 8));
-        ol |= __shfl_xor_sync(0xffffffffu, ol, 8);
+      // does an element exceed its column's exponent?
+      int over = 0;
+      if (!slow) {
+#pragma unroll
+        for (int k = 0; k < NR; k++) over |= (int)(Ecur - EOFS - field(cur, k));
+        over = over < 0;
+      } else {
+#pragma unroll
+        for (int k = 0; k < NR; k++) over |= exp_field(value(cur, k)) > Ecur;
       }
-      mh = max(mh, __shfl_xor_sync(0xffffffffu, mh, 16));
-      ol |= __shfl_xor_sync(0xffffffffu, ol, 16);
-      uint32_t e = mh >> 20;
-      if (e == 0 && (mh | ol)) e = 1;
-      __syncwarp();
+      over = __any_sync(0xffffffffu, over && cvalid);
       if (lane == 0) mbar_arrive(&raw_empty[rs]);
-      const int bump = slicers_any(e > Ecur);
-      const bool start = ls == 0 || bump || ls - pstart >= PSTAGES || epoch_periods >= MAX_EPOCH_PERIODS;
-      if (start) {
-        if (pend) {  // the period before the current one still holds its TMEM set: finish it now
-          // its last MMAs: waited on already once its slot was reused (ls >= pend_last + DSLOTS);
-          // before that the slot's barrier has not moved past that phase, so the parity wait holds
-          if (ls < pend_last + DSLOTS && lane == 0)
-            wait_ab(&dempty[pend_last % DSLOTS], (uint32_t)((pend_last / DSLOTS) & 1), abort_f, p.err);
-          __syncwarp();
-          for (int k = pend_piece; k < 4; k++) drain_piece(pend_buf, k);
-          pend = 0;
+      if (over) {  // rare: raise the exponents that are exceeded
+        uint32_t e = 0;
+#pragma unroll
+        for (int k = 0; k < NR; k++) e = max(e, exp_field(value(cur, k)));
+        if (gram) e = max(e, __shfl_xor_sync(0xffffffffu, e, 4));
+        e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
+        e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
+        // a record keeps two exponents: the drain of the periods before this warp's last raise has
+        // read what it needs (those periods ended there, whatever this stage holds)
+        for (uint32_t i = 0;; i++) {
+          int done = 1;
+#pragma unroll
+          for (int w = 0; w < DW; w++) done &= dprog[w] >= raised;
+          if (done || *abort_f) break;
+          if (i >= (1u << 22)) {
+            ok = 0;
+            break;
+          }
+          __nanosleep(64);
         }
-        if (ls > 0) {
-          pend = 1;
-          pend_buf = cur_buf;
-          pend_last = ls - 1;
-          pend_piece = 0;
+        __syncwarp();
+        if (cvalid && e > Ecur) {
+          if (sub == 0)
+            rec[(isB ? 64 : 0) + c] = ((uint64_t)(uint32_t)ls << 32) | (uint64_t)((Ecur << 16) | (e + HEAD));
+          Ecur = e + HEAD;
         }
-        cur_buf ^= 1;
-        pstart = ls;
-        if (bump || ls == 0 || epoch_periods >= MAX_EPOCH_PERIODS) {
-          epoch++;
-          epoch_periods = 0;
-        }
-        epoch_periods++;
-        if (e > Ecur) Ecur = e + HEAD;
-        if (sub == 0) {
-          rec[cur_buf * 128 + (isB ? 64 : 0) + c] = (int)Ecur;
-          if (gram) rec[cur_buf * 128 + 64 + c] = (int)Ecur;
-        }
-        if (tid == 0) rec_epoch[cur_buf] = epoch;
-      } else if (pend && ls >= pend_last + DSLOTS) {
-        // the MMAs of the pending period's last stage are complete (waited on for slot reuse)
-        drain_piece(pend_buf, pend_piece);
-        if (++pend_piece == 4) pend = 0;
+        raised = ls;
+        vflag[ls & 3] = ls + 1;
+        slow = __any_sync(0xffffffffu, Ecur <= EMIN || (F32 && Ecur > EOFS + 254 && cvalid));
       }
-      if (tid == 0) flags[ds] = (start ? 1 : 0) | (cur_buf << 1);
+      if (ls >= DSLOTS) ok &= wait_warp(&dempty[ds], dph ^ 1u, abort_f);
       // slice: digits relative to Ecur into slot ds
       unsigned char* sa = dig + (size_t)ds * SLOT;
       unsigned char* sb = sa + SLOT_A;
       if (cvalid) {
-        // digits 2 gi + 1 and 2 gi + 2 of each element pair come from one byte interleave
-        if (!gram) {
-          uint64_t g[8];
+        uint64_t g[NR];
+        if (!slow) {
 #pragma unroll
-          for (int k = 0; k < 8; k++) g[k] = fixed_g(v[k], Ecur);
-          unsigned char* dst = (isB ? sb + sub * LBO_B : sa + sub * LBO_A) + cofs;
-#pragma unroll
-          for (int gi = 0; gi < 4; gi++) {
-            uint32_t wa[4], wb[4];
-#pragma unroll
-            for (int pp = 0; pp < 4; pp++) {
-              const uint32_t x = gi < 2 ? (uint32_t)(g[2 * pp] >> 32) : (uint32_t)g[2 * pp];
-              const uint32_t y = gi < 2 ? (uint32_t)(g[2 * pp + 1] >> 32) : (uint32_t)g[2 * pp + 1];
-              const uint32_t t = __byte_perm(x, y, (gi & 1) ? 0x5140 : 0x7362);
-              wa[pp] = half_pair(t, 0x4342);
-              wb[pp] = half_pair(t, 0x4140);
-            }
-            const int d1 = 2 * gi + 1, d2 = 2 * gi + 2;
-            *reinterpret_cast<uint4*>(dst + (isB ? d1 : slot_a(d1)) * 1024) = make_uint4(wa[0], wa[1], wa[2], wa[3]);
-            *reinterpret_cast<uint4*>(dst + (isB ? d2 : slot_a(d2)) * 1024) = make_uint4(wb[0], wb[1], wb[2], wb[3]);
-          }
+          for (int k = 0; k < NR; k++)
+            g[k] = fixed_fast<TI>(cur.hi[k], cur.lo[k], Ecur - EOFS - field(cur, k));
         } else {
-          uint64_t g[4];
 #pragma unroll
-          for (int k = 0; k < 4; k++) g[k] = fixed_g(v[k], Ecur);
-          unsigned char* da = sa + (sub >> 1) * LBO_A + cofs + (sub & 1) * 8;
-          unsigned char* db = sb + (sub >> 1) * LBO_B + cofs + (sub & 1) * 8;
+          for (int k = 0; k < NR; k++) g[k] = fixed_g(value(cur, k), Ecur);
+        }
+        // digits d = 2 gi + 1 and d + 1 of each element pair come from one byte interleave
+        auto digits = [&](int gi, uint32_t (&w1)[NR / 2], uint32_t (&w2)[NR / 2]) {
+#pragma unroll
+          for (int pp = 0; pp < NR / 2; pp++) {
+            const uint32_t x = gi < 2 ? (uint32_t)(g[2 * pp] >> 32) : (uint32_t)g[2 * pp];
+            const uint32_t y = gi < 2 ? (uint32_t)(g[2 * pp + 1] >> 32) : (uint32_t)g[2 * pp + 1];
+            const uint32_t t = __byte_perm(x, y, (gi & 1) ? 0x5140 : 0x7362);
+            w1[pp] = half_pair(t, 0x4342);
+            w2[pp] = half_pair(t, 0x4140);
+          }
+        };
+        if (GR == 1 || (GR == 2 && gram)) {
+          unsigned char* da = sa + (sub >> 2) * LBO_A + cofs + (sub & 3) * 4;
+          unsigned char* db = sb + (sub >> 2) * LBO_B + cofs + (sub & 3) * 4;
 #pragma unroll
           for (int gi = 0; gi < 4; gi++) {
-            uint32_t wa[2], wb[2];
+            uint32_t w1[NR / 2], w2[NR / 2];
+            digits(gi, w1, w2);
+            const int d = 2 * gi + 1;
+            *reinterpret_cast<uint32_t*>(da + slot_a(d) * 1024) = w1[0];
+            *reinterpret_cast<uint32_t*>(db + d * 1024) = w1[0];
+            *reinterpret_cast<uint32_t*>(da + slot_a(d + 1) * 1024) = w2[0];
+            *reinterpret_cast<uint32_t*>(db + (d + 1) * 1024) = w2[0];
+          }
+        } else if constexpr (NR == 4) {
+          unsigned char* dst = (isB ? sb + (sub >> 1) * LBO_B : sa + (sub >> 1) * LBO_A) + cofs + (sub & 1) * 8;
 #pragma unroll
-            for (int pp = 0; pp < 2; pp++) {
-              const uint32_t x = gi < 2 ? (uint32_t)(g[2 * pp] >> 32) : (uint32_t)g[2 * pp];
-              const uint32_t y = gi < 2 ? (uint32_t)(g[2 * pp + 1] >> 32) : (uint32_t)g[2 * pp + 1];
-              const uint32_t t = __byte_perm(x, y, (gi & 1) ? 0x5140 : 0x7362);
-              wa[pp] = half_pair(t, 0x4342);
-              wb[pp] = half_pair(t, 0x4140);
-            }
-            const int d1 = 2 * gi + 1, d2 = 2 * gi + 2;
-            *reinterpret_cast<uint2*>(da + slot_a(d1) * 1024) = make_uint2(wa[0], wa[1]);
-            *reinterpret_cast<uint2*>(db + d1 * 1024) = make_uint2(wa[0], wa[1]);
-            *reinterpret_cast<uint2*>(da + slot_a(d2) * 1024) = make_uint2(wb[0], wb[1]);
-            *reinterpret_cast<uint2*>(db + d2 * 1024) = make_uint2(wb[0], wb[1]);
+          for (int gi = 0; gi < 4; gi++) {
+            uint32_t w1[NR / 2], w2[NR / 2];
+            digits(gi, w1, w2);
+            const int d = 2 * gi + 1;
+            *reinterpret_cast<uint2*>(dst + (isB ? d : slot_a(d)) * 1024) = make_uint2(w1[0], w1[1]);
+            *reinterpret_cast<uint2*>(dst + (isB ? d + 1 : slot_a(d + 1)) * 1024) = make_uint2(w2[0], w2[1]);
           }
         }
       }
       fence_proxy_async_smem();
-      tc_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&dfull[ds]);
-    }
-    // last periods
-    if (pend) {
-      if (nst - 1 < pend_last + DSLOTS && lane == 0)  // no processed stage reused its slot
-        wait_ab(&dempty[pend_last % DSLOTS], (uint32_t)((pend_last / DSLOTS) & 1), abort_f, p.err);
-      __syncwarp();
-      for (int k = pend_piece; k < 4; k++) drain_piece(pend_buf, k);
-    }
-    if (nst > 0) {
-      if (lane == 0)
-        wait_ab(&dempty[(nst - 1) % DSLOTS], (uint32_t)(((nst - 1) / DSLOTS) & 1), abort_f, p.err);
-      __syncwarp();
-      for (int k = 0; k < 4; k++) drain_piece(cur_buf, k);
-    }
-    flush();
-    // the CTA's sum of a cell: levels 2..5 (half 0) plus levels 6..9 (half 1), into half 0; with
-    // folded stages the second row half's quadrant is then added to the first's
-    slicers_sync();
-    if (hm == 0 && live && mv < Mb)
-      for (int x = 0; x < 32; x++) {
-        const int n = 32 * nh + x;
-        if (n - nofs < Nb) part[n * 64 + m] += part[4096 + n * 64 + m];
+      if (!__all_sync(0xffffffffu, ok)) {  // a wait ran out, here or in another warp
+        *abort_f = 1;
+        if (lane == 0) atomicExch(p.err, SKINNY_DEVERR_TIMEOUT);
+        break;
       }
-    if constexpr (FOLD) {
-      slicers_sync();
-      if (hm == 0 && nh == 0 && q == 0 && m < Mb)
-        for (int x = 0; x < Nb; x++) part[x * 64 + m] += part[(x + 32) * 64 + m + 32];
     }
   }
 
   tc_before();
   __syncthreads();
+  // back to the registers of the launch (a warpgroup's warps have met since the first change)
+  if (warp >= SW && warp < WPROD)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  else
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
   if (*abort_f) return;
+
+  // the CTA's sum of a cell: levels 2..5 (half 0) plus levels 6..9 (half 1), into half 0; with
+  // folded stages plus the second row half's quadrant
+  double* part = p.partials + (size_t)(blk * nchunks + chunk) * 8192;
+  for (int e = tid; e < Mb * Nb; e += THREADS) {
+    const int cell = (e / Mb) * 64 + e % Mb;
+    double v = part[cell] + part[4096 + cell];
+    if (FOLD) v += part[cell + 32 * 64 + 32] + part[4096 + cell + 32 * 64 + 32];
+    part[cell] = v;
+  }
 
   // ---- cross-CTA finish, two levels: the last CTA of each group of GROUP chunks sums the group's
   // partials in chunk order; the last group to finish sums the group sums in group order and
@@ -653,7 +793,8 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
     double sum = 0.0;
 #pragma unroll
     for (int i = 0; i < 15; i++) sum += v[i];
-    const int64_t ci = (int64_t)(W * bj + nn) * p.ldc + W * bi + mm, cmi = (int64_t)(W * bi + mm) * p.ldc + W * bj + nn;
+    const int64_t ci = (int64_t)(W * bj + nn) * p.ldc + W * bi + mm;
+    const int64_t cmi = (int64_t)(W * bi + mm) * p.ldc + W * bj + nn;
     const bool mirror = p.sym && bi < bj;  // Gram: the mirrored block holds the same sums
     if (p.out_f32) {  // the one rounding of an FP32 result
       float* C = static_cast<float*>(p.C);
@@ -738,15 +879,24 @@ skinny_status split_wide_t(skinny_handle h, bool in_f32, bool out_f32, int64_t M
   a.partials = (double*)ws.partials;
   a.counter = ws.counter;
   a.err = h->err;
-  static SmemAttr attr[4];
+  static SmemAttr attr[12];
   auto launch = [&](auto kernel, SmemAttr& at) {
     ensure_smem_attr(kernel, smem, at);
     kernel<<<(int)grid, THREADS, smem, st>>>(a);
   };
-  if (!in_f32)
-    fold ? launch(split_wide_kernel<double, true>, attr[0]) : launch(split_wide_kernel<double, false>, attr[1]);
-  else
-    fold ? launch(split_wide_kernel<float, true>, attr[2]) : launch(split_wide_kernel<float, false>, attr[3]);
+  const int gk = !a.sym ? 0 : (a.nblk == 1 ? 1 : 2);  // folded products have one block
+#define SK_WIDE(T, I)                                                                                 \
+  {                                                                                                   \
+    if (fold)                                                                                         \
+      gk ? launch(split_wide_kernel<T, true, 1>, attr[I]) : launch(split_wide_kernel<T, true, 0>, attr[I + 1]); \
+    else if (gk == 0)                                                                                 \
+      launch(split_wide_kernel<T, false, 0>, attr[I + 2]);                                            \
+    else                                                                                              \
+      gk == 1 ? launch(split_wide_kernel<T, false, 1>, attr[I + 3])                                   \
+              : launch(split_wide_kernel<T, false, 2>, attr[I + 4]);                                  \
+  }
+  if (!in_f32) SK_WIDE(double, 0) else SK_WIDE(float, 6)
+#undef SK_WIDE
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
