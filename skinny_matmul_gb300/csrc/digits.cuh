@@ -14,45 +14,61 @@ namespace skinny {
 constexpr int NDIGITS = 8;
 
 // G = F + 0x8080...80 for the 62-bit fixed-point magnitude F of x relative to exponent field E:
-// byte i of G (most significant first) is digit i + 128, so the digits are balanced
-__device__ __forceinline__ void g_words(double x, uint32_t E, uint32_t& gh, uint32_t& gl, bool& neg) {
+// byte i of G (most significant first) is digit i + 128, so the digits are balanced.
+// FAST: E > EMIN_FAST, where zeros and subnormal numbers shift out entirely and need no case of their own
+constexpr uint32_t EMIN_FAST = 64;
+template <bool FAST = false>
+__device__ __forceinline__ void g_words(double x, uint32_t E, uint32_t& gh, uint32_t& gl) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
   const uint32_t ef = (hi >> 20) & 0x7FF;
-  neg = (hi >> 31) != 0;
-  const uint32_t eff = ef ? ef : 1u;
-  const uint64_t mant = ((uint64_t)((hi & 0xFFFFFu) | (ef ? 0x100000u : 0u)) << 32) | lo;
-  const uint32_t sh = E - eff;
-  const uint64_t F = sh < 64 ? ((mant << 9) >> sh) : 0ull;
+  uint64_t F;
+  if constexpr (FAST) {
+    const uint64_t m9 =
+        ((uint64_t)__funnelshift_l(lo, (hi & 0xFFFFFu) | 0x100000u, 9) << 32) | (uint64_t)(uint32_t)(lo << 9);
+    asm("shr.u64 %0, %1, %2;" : "=l"(F) : "l"(m9), "r"(E - ef));  // 0 from 64 on
+  } else {
+    const uint32_t eff = ef ? ef : 1u;
+    const uint64_t mant = ((uint64_t)((hi & 0xFFFFFu) | (ef ? 0x100000u : 0u)) << 32) | lo;
+    const uint32_t sh = E - eff;
+    F = sh < 64 ? ((mant << 9) >> sh) : 0ull;
+  }
   const uint64_t G = F + 0x8080808080808080ull;
   gh = (uint32_t)(G >> 32);
   gl = (uint32_t)G;
 }
 
-// The eight FP16 digit pairs of elements a, b (a in the low halves), digit i in out[i].  A byte g
-// of G becomes the half 1024 + g by pairing it with the byte 0x64 (two byte permutes), and one
-// HFMA2 subtracts 1152 and applies each element's sign: (1024 + g - 1152) * s = (g - 128) * s,
-// exact in FP16.  About 1.25 instructions per digit.
-__device__ __forceinline__ void digit_pairs(uint32_t gha, uint32_t gla, bool na, uint32_t ghb, uint32_t glb, bool nb,
-                                            uint32_t (&out)[NDIGITS]) {
-  const __half2 s = __halves2half2(na ? __float2half(-1.0f) : __float2half(1.0f),
-                                   nb ? __float2half(-1.0f) : __float2half(1.0f));
-  const __half2 c = __hmul2(s, __float2half2_rn(-1152.0f));
-  auto dig = [&](uint32_t pair, uint32_t sel) {
+// signs of elements a, b as FP16 factors (a in the low half), and -1152 times them
+struct SignPair {
+  uint32_t s, c;
+};
+__device__ __forceinline__ SignPair sign_pair(double a, double b) {
+  const uint32_t t = __byte_perm((uint32_t)__double2hiint(a), (uint32_t)__double2hiint(b), 0x7632) & 0x80008000u;
+  return {t | 0x3C003C00u, t ^ 0xE480E480u};
+}
+// Two FP16 digit pairs of elements a, b (a in the low halves) from one 32-bit word of their G's: the
+// digits of its upper (half 0) or lower bytes, the higher one in d0.  A byte g of G becomes the half
+// 1024 + g by pairing it with the byte 0x64, and one HFMA2 subtracts 1152 and applies each element's
+// sign: (1024 + g - 1152) * s = (g - 128) * s, exact in FP16.  1.25 instructions a digit.
+__device__ __forceinline__ void digit_pairs2(uint32_t ga, uint32_t gb, int lower, SignPair sg, uint32_t& d0,
+                                             uint32_t& d1) {
+  const uint32_t pair = __byte_perm(ga, gb, lower ? 0x4051 : 0x6273);  // [a.b1, b.b1, a.b0, b.b0] or the upper bytes
+  auto dig = [&](uint32_t sel) {
     const uint32_t u = __byte_perm(pair, 0x64646464u, sel);
-    __half2 h = *reinterpret_cast<const __half2*>(&u);
-    h = __hfma2(h, s, c);
+    const __half2 h = __hfma2(*reinterpret_cast<const __half2*>(&u), *reinterpret_cast<const __half2*>(&sg.s),
+                              *reinterpret_cast<const __half2*>(&sg.c));
     return *reinterpret_cast<const uint32_t*>(&h);
   };
-#pragma unroll
-  for (int w = 0; w < 2; w++) {
-    const uint32_t ga = w ? gla : gha, gb = w ? glb : ghb;
-    const uint32_t x01 = __byte_perm(ga, gb, 0x6273);  // [a.b3, b.b3, a.b2, b.b2]
-    const uint32_t x23 = __byte_perm(ga, gb, 0x4051);  // [a.b1, b.b1, a.b0, b.b0]
-    out[4 * w + 0] = dig(x01, 0x4140);
-    out[4 * w + 1] = dig(x01, 0x4342);
-    out[4 * w + 2] = dig(x23, 0x4140);
-    out[4 * w + 3] = dig(x23, 0x4342);
-  }
+  d0 = dig(0x4140);
+  d1 = dig(0x4342);
+}
+
+// the eight digit pairs, digit i in out[i]
+__device__ __forceinline__ void digit_pairs(uint32_t gha, uint32_t gla, uint32_t ghb, uint32_t glb, SignPair sg,
+                                            uint32_t (&out)[NDIGITS]) {
+  digit_pairs2(gha, ghb, 0, sg, out[0], out[1]);
+  digit_pairs2(gha, ghb, 1, sg, out[2], out[3]);
+  digit_pairs2(gla, glb, 0, sg, out[4], out[5]);
+  digit_pairs2(gla, glb, 1, sg, out[6], out[7]);
 }
 
 }  // namespace skinny

@@ -18,21 +18,27 @@
 //   * |d_i d_j| <= 2^14, so over a period of <= 1024 rows every partial sum is an integer of
 //     magnitude <= 2^24: the FP32 accumulation in TMEM is exact.  Two accumulator sets alternate
 //     between periods, so the drain of one period runs while the MMAs of the next proceed.
-//   * Drain: TMEM -> int32; level sums S_L = sum_{i+j=L} D_ij (L = 2..9) are formed with a
-//     per-lane rotation and warp shuffles (all eight levels per shuffle stage), then in shared
-//     memory with integer atomics;
+//   * Drain: TMEM -> int32, added per digit pair (i, j) in registers over up to 15 periods of the same
+//     exponents (8 * 15 * 2^24 < 2^31); then a few columns of C at a time pass through shared memory
+//     and one thread forms the level sums S_L = sum_{i+j=L} D_ij (L = 2..9) of a cell;
 //     V = sum_L S_L 2^(8(16-L)) is assembled from two int64 words and added to an FP64
 //     accumulator per C entry with weight 2^(EA+EB-2168).  Levels L >= 10 are dropped: their
 //     weight is below 2^-56 of the leading level (2^-52 with the headroom).
 //   * Warp roles, hand-offs through mbarriers (no CTA-wide barrier while streaming):
-//       warps 0-7  slicers: per round of rr rows (rr * (M + N) / 8 units of one column and 8 rows,
-//                  at most two per thread) read the FP64 values from the stage ring (or from
+//       warps 0-15 slicers: per round of rr rows (rr * (M + N) / 8 units of one column and 8 rows,
+//                  at most one per thread) read the FP64 values from the stage ring (or from
 //                  global memory where rows are not 16-byte aligned), check them against the
 //                  column exponents (one named barrier per round; two more only when a period
 //                  starts), slice them into a digit stage;
-//       warps 8-11 drain: one TMEM lane quadrant each;
-//       warp 12    producer: whole rounds of rows by 1-D TMA bulk copies into the FP64 ring;
-//       warp 13    MMA issuer: rr/16 MMAs per round into the period's accumulator set.
+//       warps 16-19 drain: one TMEM lane quadrant each;
+//       warp 20    producer: whole rounds of rows by 1-D TMA bulk copies into the FP64 ring;
+//       warp 21    MMA issuer: rr/16 MMAs per round into the period's accumulator set.
+//     Bound: at 8 x 8 a round of 256 rows takes ~3500 clocks.  Of these the ALU pipe needs ~1100 for
+//     the digits, the tensor pipe 640 and shared memory 1800, but the phases of a round (read, vote on
+//     the exponents, slice) follow one another in all warps at once.  With 8 slicer warps of two units
+//     a thread it was ~5400, and the drain sorted every period by level with shuffles and atomics
+//     (8000 clocks a period, of which the last one's was not hidden).  Measured f64 8 x 8: K = 2^20
+//     90 -> 64 us, K = 2^14 16.7 -> 14.8; 16 x 16, K = 2^20: 166 -> 118; Gram 16: 111 -> 72.
 //     The roles that wait most of the time (drain, producer, MMA) sleep between polls, so that
 //     their polling leaves issue slots to the slicers.  Every wait is bounded; a wait that runs
 //     out sets the error word, every role stops at its next wait, and the CTA writes no C.
@@ -51,18 +57,23 @@ namespace skinny {
 namespace split {
 
 constexpr int PERIOD = 1024;   // rows accumulated exactly in TMEM (|sum| <= 1024 * 2^14)
+constexpr int MAXSUM = 15;     // periods summed before the levels are (8 pairs * 15 * 2^24 < 2^31)
 constexpr int DIGITS = 8;
-constexpr int NSLICE = 8;      // slicer warps 0-7
-constexpr int NDRAIN = 4;      // drain warps 8-11 (one TMEM lane quadrant each)
+constexpr int NSLICE = 16;     // slicer warps 0-15
+constexpr int NDRAIN = 4;      // drain warps 16-19 (one TMEM lane quadrant each)
 constexpr int WPROD = NSLICE + NDRAIN, WMMA = WPROD + 1;
-constexpr int THREADS = (WMMA + 1) * 32;  // 448
+// six warpgroups (the last one: producer, MMA issuer, two idle warps) launched with 80 registers a
+// thread, of which the last group gives back 40 and the slicers 8 for the drain warps' 152
+constexpr int THREADS = (WMMA + 3) * 32;
 constexpr int SLICERS = NSLICE * 32;
 constexpr int HEAD = 2;        // exponent headroom granted when a column's exponent is raised
 constexpr int MAXST = 4;       // FP64 stages (at most)
 constexpr int MAXDST = 3;      // digit stages (at most)
 constexpr int DPAD = 128 * 16; // slack after an A digit buffer: the MMA reads 128 rows per k-octet
 constexpr int HDR = 2048;      // barriers, TMEM slot, round and period records, exponents
-constexpr int SBYTES = 8 * 16 * 16 * 4;  // level sums S[8][16][16]
+constexpr int NCMAX = 4;                 // columns of B whose digit pairs the drain sorts by level at a time
+constexpr int DSTRIDE = 128 + 8;
+constexpr int SBYTES = DIGITS * NCMAX * DSTRIDE * 4;
 constexpr int CBYTES = 256 * 8;          // FP64 accumulators of the C entries
 constexpr int STATIC_RESERVE = 1024;     // the kernel's static shared memory
 constexpr uint32_t SLEEP_DRAIN = 256;    // ns between polls of the drain warps (a period is ~8 rounds)
@@ -153,25 +164,25 @@ __device__ __forceinline__ double pow2i(int e) {  // 2^e for e in [-1022, 1023],
   return __hiloint2double((e + 1023) << 20, 0);
 }
 
-// Slice one unit: 8 consecutive rows (octet o) of column c into the digit buffer `buf`
-// (rows (i-1)*CP + c), relative to exponent E.  FP16 digits formed from the bytes of G with byte
-// permutes and one HFMA2 per digit pair (digits.cuh).
-__device__ __forceinline__ void slice_unit(const double (&v)[8], uint32_t E, int c, int CP, int o,
-                                           uint32_t lbo, unsigned char* buf) {
-  uint32_t dp[4][NDIGITS];  // row pairs (0,1), (2,3), (4,5), (6,7) of the octet
+// Slice one unit: 8 consecutive rows of column c into the octet `buf` of a digit buffer
+// (rows (i-1)*CP + c), relative to exponent E (FAST: E > EMIN_FAST).  FP16 digits formed from the bytes of G with byte
+// permutes and one HFMA2 per digit pair (digits.cuh), stored as they are formed.
+template <bool FAST>
+__device__ __forceinline__ void slice_unit(const double (&v)[8], uint32_t E, int c, int CP, unsigned char* buf) {
+  uint32_t gw[2][8];
+  SignPair sg[4];  // row pairs (0,1), (2,3), (4,5), (6,7) of the octet
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    uint32_t gha, gla, ghb, glb;
-    bool na, nb;
-    g_words(v[2 * q], E, gha, gla, na);
-    g_words(v[2 * q + 1], E, ghb, glb, nb);
-    digit_pairs(gha, gla, na, ghb, glb, nb, dp[q]);
-  }
+  for (int q = 0; q < 8; q++) g_words<FAST>(v[q], E, gw[0][q], gw[1][q]);
 #pragma unroll
-  for (int i = 0; i < DIGITS; i++) {
-    const int r = i * CP + c;
-    *reinterpret_cast<uint4*>(buf + o * lbo + (r >> 3) * 128 + (r & 7) * 16) =
-        make_uint4(dp[0][i], dp[1][i], dp[2][i], dp[3][i]);
+  for (int q = 0; q < 4; q++) sg[q] = sign_pair(v[2 * q], v[2 * q + 1]);
+#pragma unroll
+  for (int i = 0; i < DIGITS; i += 2) {
+    uint32_t d0[4], d1[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) digit_pairs2(gw[i / 4][2 * q], gw[i / 4][2 * q + 1], i & 2, sg[q], d0[q], d1[q]);
+    const int r0 = i * CP + c, r1 = r0 + CP;
+    *reinterpret_cast<uint4*>(buf + (r0 >> 3) * 128 + (r0 & 7) * 16) = make_uint4(d0[0], d0[1], d0[2], d0[3]);
+    *reinterpret_cast<uint4*>(buf + (r1 >> 3) * 128 + (r1 & 7) * 16) = make_uint4(d1[0], d1[1], d1[2], d1[3]);
   }
 }
 
@@ -182,9 +193,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 __device__ __forceinline__ int slicers_any(int pred) {
   int r;
   asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, 1, 256, p;\n selp.s32 %0, 1, 0, q;\n}\n"
+      "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n selp.s32 %0, 1, 0, q;\n}\n"
       : "=r"(r)
-      : "r"(pred)
+      : "r"(pred), "n"(SLICERS)
       : "memory");
   return r;
 }
@@ -198,19 +209,6 @@ __device__ __forceinline__ int drainers_any(int pred) {
   return r;
 }
 __device__ __forceinline__ void drainers_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
-
-// Sum of c[t] over the lanes that hold the same column m of A (lane = (i0, m), MP lanes per
-// digit): xor-shuffles at distances MP..16, the eight levels' shuffles of a stage issued together
-// so that their latencies overlap.
-__device__ __forceinline__ void level_reduce(int (&c)[DIGITS], int MP) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    if (o >= MP) {  // warp-uniform
-#pragma unroll
-      for (int t = 0; t < DIGITS; t++) c[t] += __shfl_xor_sync(0xffffffffu, c[t], o);
-    }
-  }
-}
 
 // bounded wait that also gives up as soon as another thread of the CTA has given up; sleep_ns
 // between polls for the roles that wait most of the time
@@ -230,6 +228,7 @@ template <int NP, typename TI>
 __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p) {
   constexpr int BN = NP < 8 ? NP : 8;  // B columns per drain block
   constexpr int NB = NP / BN;          // drain blocks
+  constexpr int NC = NP < NCMAX ? NP : NCMAX;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);           // [MAXST] FP64 stage landed
   uint64_t* empty = full + MAXST;                                // [MAXST] FP64 stage consumed
@@ -243,9 +242,11 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
   volatile int* abort_f = reinterpret_cast<volatile int*>(smem + 196);
   volatile int* rinfo = reinterpret_cast<volatile int*>(smem + 208);  // [MAXDST] period | first << 30
   volatile int* plast = reinterpret_cast<volatile int*>(smem + 224);  // [2] the period is the last
+  volatile int* pchg = reinterpret_cast<volatile int*>(smem + 232);  // [2] the period's exponents are new
   int* Ecur = reinterpret_cast<int*>(smem + 256);                      // [32] A columns, then B
   int* pe = reinterpret_cast<int*>(smem + 384);                        // [2][32] a period's exponents
-  int* S = reinterpret_cast<int*>(smem + HDR);
+  int* ae = reinterpret_cast<int*>(smem + 640);                        // [32] exponents of the drain's sums
+  int* D = reinterpret_cast<int*>(smem + HDR);                         // [8 * NC][DSTRIDE]
   double* cacc = reinterpret_cast<double*>(smem + HDR + SBYTES);
   unsigned char* ring = smem + HDR + SBYTES + CBYTES;
   unsigned char* dig = ring + (size_t)p.stages * p.stage_bytes;  // 1024-aligned by the host
@@ -279,14 +280,13 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
     for (int i = 0; i < 2; i++) {
       mbar_init(&pdone[i], 1);
       mbar_init(&pfin[i], 1);
-      mbar_init(&drained[i], 1);
+      mbar_init(&drained[i], NDRAIN);
     }
     mbar_init(bar_fin, 1);
     *abort_f = 0;
     fence_mbar_init();
   }
   if (tid < 32) Ecur[tid] = 0;
-  for (int e = tid; e < SBYTES / 4; e += THREADS) S[e] = 0;
   for (int e = tid; e < CBYTES / 8; e += THREADS) cacc[e] = 0.0;
   // padding rows of the digit stages stay zero: clear every stage once
   for (uint32_t o = tid * 16; o < (uint32_t)DST * (p.dig_a + p.dig_b); o += THREADS * 16)
@@ -297,277 +297,285 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
   tc_fence_after();
   const uint32_t tmem = *tslot;
 
-  if (warp == WPROD) {
-    // ---- producer: whole rounds of rows of A and B into the FP64 stage ring ----------------------
-    int issued = 0;
-    for (int t = 0; t < nt; t++) {
-      const int s = t % p.stages, use = t / p.stages;
-      if (use > 0) {
-        int ok = 0;
-        if (lane == 0) ok = wait_ab(&empty[s], (uint32_t)((use - 1) & 1), abort_f, p.err, SLEEP_PRODUCER);
-        if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      }
-      if (lane == 0) {
-        const int64_t tt = t_begin + t;
-        if (is_bulk(tt)) {
-          const int64_t r0 = tt * p.rr;
-          constexpr uint32_t ES = sizeof(TI);
-          const uint32_t ba = (uint32_t)(p.rr * p.lda * ES), bb = p.gram ? 0u : (uint32_t)(p.rr * p.ldb * ES);
-          unsigned char* st = ring + (size_t)s * p.stage_bytes;
-          mbar_arrive_expect_tx(&full[s], ba + bb);
-          bulk_g2s(st, static_cast<const TI*>(p.A) + r0 * p.lda, ba, &full[s]);
-          if (!p.gram) bulk_g2s(st + p.tile_a, static_cast<const TI*>(p.B) + r0 * p.ldb, bb, &full[s]);
-        } else {
-          mbar_arrive(&full[s]);  // no copy: the slicers read this round from global memory
-        }
-      }
-      issued = t + 1;
-    }
-    // copies in flight land before the CTA ends
-    if (lane == 0)
-      for (int t = max(0, issued - p.stages); t < issued; t++)
-        mbar_wait_bounded(&full[t % p.stages], (uint32_t)((t / p.stages) & 1), nullptr);
-  } else if (warp == WMMA) {
-    // ---- MMA issuer -------------------------------------------------------------------------------
-    if (lane == 0) {
-      // idesc: D f32, A/B f16, K-major both, N = nmma, M = 128
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(p.nmma >> 3) << 17) | ((128u >> 4) << 24);
-      const uint32_t lbb = p.gram ? p.lbo_a : p.lbo_b;
-      int pcur = -1, issued = 0;
-      bool ok = true;
+  if (warp >= WPROD) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == WPROD) {
+      // ---- producer: whole rounds of rows of A and B into the FP64 stage ring ----------------------
+      int issued = 0;
       for (int t = 0; t < nt; t++) {
-        const int d = t % DST;
-        if (!wait_ab(&dfull[d], (uint32_t)((t / DST) & 1), abort_f, p.err, SLEEP_MMA)) {
-          ok = false;
-          break;
+        const int s = t % p.stages, use = t / p.stages;
+        if (use > 0) {
+          int ok = 0;
+          if (lane == 0) ok = wait_ab(&empty[s], (uint32_t)((use - 1) & 1), abort_f, p.err, SLEEP_PRODUCER);
+          if (!__shfl_sync(0xffffffffu, ok, 0)) break;
         }
-        tc_fence_after();
-        const int info = rinfo[d];
-        const int pp = info & 0x3FFFFFFF;
-        const bool first = (info >> 30) & 1;
-        if (first) {
-          if (pp >= 1) {  // the previous period is complete once its MMAs finish
-            mma_commit(&pdone[(pp - 1) & 1]);
-            plast[(pp - 1) & 1] = 0;
-            mbar_arrive(&pfin[(pp - 1) & 1]);
+        if (lane == 0) {
+          const int64_t tt = t_begin + t;
+          if (is_bulk(tt)) {
+            const int64_t r0 = tt * p.rr;
+            constexpr uint32_t ES = sizeof(TI);
+            const uint32_t ba = (uint32_t)(p.rr * p.lda * ES), bb = p.gram ? 0u : (uint32_t)(p.rr * p.ldb * ES);
+            unsigned char* st = ring + (size_t)s * p.stage_bytes;
+            mbar_arrive_expect_tx(&full[s], ba + bb);
+            bulk_g2s(st, static_cast<const TI*>(p.A) + r0 * p.lda, ba, &full[s]);
+            if (!p.gram) bulk_g2s(st + p.tile_a, static_cast<const TI*>(p.B) + r0 * p.ldb, bb, &full[s]);
+          } else {
+            mbar_arrive(&full[s]);  // no copy: the slicers read this round from global memory
           }
-          if (pp >= 2) {  // this period's accumulator set was drained (period pp - 2)
-            if (!wait_ab(&drained[pp & 1], (uint32_t)(((pp - 2) >> 1) & 1), abort_f, p.err, SLEEP_MMA)) {
-              ok = false;
-              break;
+        }
+        issued = t + 1;
+      }
+      // copies in flight land before the CTA ends
+      if (lane == 0)
+        for (int t = max(0, issued - p.stages); t < issued; t++)
+          mbar_wait_bounded(&full[t % p.stages], (uint32_t)((t / p.stages) & 1), nullptr);
+    } else if (warp == WMMA) {
+      // ---- MMA issuer -------------------------------------------------------------------------------
+      if (lane == 0) {
+        // idesc: D f32, A/B f16, K-major both, N = nmma, M = 128
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(p.nmma >> 3) << 17) | ((128u >> 4) << 24);
+        const uint32_t lbb = p.gram ? p.lbo_a : p.lbo_b;
+        int pcur = -1, issued = 0;
+        bool ok = true;
+        for (int t = 0; t < nt; t++) {
+          const int d = t % DST;
+          if (!wait_ab(&dfull[d], (uint32_t)((t / DST) & 1), abort_f, p.err, SLEEP_MMA)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const int info = rinfo[d];
+          const int pp = info & 0x3FFFFFFF;
+          const bool first = (info >> 30) & 1;
+          if (first) {
+            if (pp >= 1) {  // the previous period is complete once its MMAs finish
+              mma_commit(&pdone[(pp - 1) & 1]);
+              plast[(pp - 1) & 1] = 0;
+              mbar_arrive(&pfin[(pp - 1) & 1]);
             }
-            tc_fence_after();
+            if (pp >= 2) {  // this period's accumulator set was drained (period pp - 2)
+              if (!wait_ab(&drained[pp & 1], (uint32_t)(((pp - 2) >> 1) & 1), abort_f, p.err, SLEEP_MMA)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+            }
           }
+          const uint32_t a0 = smem_u32(digA(d)), b0 = smem_u32(digB(d));
+          const uint32_t dcol = tmem + (uint32_t)((pp & 1) * p.nmma);
+          const int ksteps = p.rr / 16;
+          uint64_t da = make_desc(a0, p.lbo_a), db = make_desc(b0, lbb);
+          for (int ks = 0; ks < ksteps; ks++) {
+            mma_f16(dcol, da, db, idesc, (first && ks == 0) ? 0u : 1u);
+            da += (2 * p.lbo_a) >> 4;  // the next two k-octets
+            db += (2 * lbb) >> 4;
+          }
+          mma_commit(&dempty[d]);
+          pcur = pp;
+          issued++;
         }
-        const uint32_t a0 = smem_u32(digA(d)), b0 = smem_u32(digB(d));
-        const uint32_t dcol = tmem + (uint32_t)((pp & 1) * p.nmma);
-        const int ksteps = p.rr / 16;
-        for (int ks = 0; ks < ksteps; ks++)
-          mma_f16(dcol, make_desc(a0 + 2 * ks * p.lbo_a, p.lbo_a), make_desc(b0 + 2 * ks * lbb, lbb), idesc,
-                   (first && ks == 0) ? 0u : 1u);
-        mma_commit(&dempty[d]);
-        pcur = pp;
-        issued++;
-      }
-      if (ok && pcur >= 0) {
-        mma_commit(&pdone[pcur & 1]);
-        plast[pcur & 1] = 1;
-        mbar_arrive(&pfin[pcur & 1]);
-      }
-      if (issued) {  // every MMA has finished before the TMEM is released
-        mma_commit(bar_fin);
-        mbar_wait_bounded(bar_fin, 0, nullptr);
+        if (ok && pcur >= 0) {
+          mma_commit(&pdone[pcur & 1]);
+          plast[pcur & 1] = 1;
+          mbar_arrive(&pfin[pcur & 1]);
+        }
+        if (issued) {  // every MMA has finished before the TMEM is released
+          mma_commit(bar_fin);
+          mbar_wait_bounded(bar_fin, 0, nullptr);
+        }
       }
     }
   } else if (warp >= NSLICE) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
     // ---- drain: a period's TMEM set -> level sums -> FP64 accumulators ---------------------------
     const int q = warp - NSLICE;        // TMEM lane quadrant
     const int dtid = tid - SLICERS;     // 0..127
     const int r = 32 * q + lane;        // TMEM lane = A digit row
-    const int i0 = r / MP, m = r - i0 * MP;  // digit index (0-based) and column of A
-    const bool rvalid = (i0 < DIGITS) && (m < M);
-    for (int pp = 0; nt > 0; pp++) {  // K = 0: no rounds, no periods
+    const bool qvalid = 32 * q < DIGITS * MP;  // quadrants without a digit row have nothing to drain
+    // Sums of the digit pairs (i0, j) of this lane's row over the periods since the exponents last
+    // changed (MAXSUM at most): one conversion and one addition per value and period
+    int acc[DIGITS * NP];
+#pragma unroll
+    for (int x = 0; x < DIGITS * NP; x++) acc[x] = 0;
+    int cnt = 0;
+    bool done = nt == 0;  // K = 0: no rounds, no periods
+    for (int pp = 0;; pp++) {
       const int set = pp & 1;
-      const uint32_t par = (uint32_t)((pp >> 1) & 1);
-      // one lane per warp polls (sleeping in between); the warp follows
-      int ok = 1;
-      if (lane == 0) {
-        ok = wait_ab(&pfin[set], par, abort_f, p.err, SLEEP_DRAIN);
-        if (ok) ok = wait_ab(&pdone[set], par, abort_f, p.err, SLEEP_DRAIN);
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (drainers_any(!ok)) break;
-      tc_fence_after();
-      const bool last = plast[set] != 0;
-      // quadrants holding no digit row (8 * MP <= 32 q) have nothing to drain
-      for (int nb = 0; nb < (32 * q < DIGITS * MP ? NB : 0); nb++) {
-        uint32_t raw[DIGITS][BN];
-#pragma unroll
-        for (int j = 0; j < DIGITS; j++) {
-          uint32_t tmp[BN];
-          tmem_ld<BN>(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(set * p.nmma + j * NP + nb * BN), tmp);
-#pragma unroll
-          for (int x = 0; x < BN; x++) raw[j][x] = tmp[x];
+      bool chg = false, last = false;
+      if (!done) {
+        const uint32_t par = (uint32_t)((pp >> 1) & 1);
+        // one lane per warp polls (sleeping in between); the warp follows
+        int ok = 1;
+        if (lane == 0) {
+          ok = wait_ab(&pfin[set], par, abort_f, p.err, SLEEP_DRAIN);
+          if (ok) ok = wait_ab(&pdone[set], par, abort_f, p.err, SLEEP_DRAIN);
         }
-        tmem_wait_ld();
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (drainers_any(!ok)) break;
+        tc_fence_after();
+        last = plast[set] != 0;
+        chg = pchg[set] != 0;
+      }
+      if (cnt && (done || chg || cnt == MAXSUM)) {  // levels -> FP64 accumulators
+        // a few columns n at a time through shared memory; a thread then forms the eight level sums of a cell
 #pragma unroll
-        for (int x = 0; x < BN; x++) {
-          const int n = nb * BN + x;
-          int R[DIGITS];
+        for (int n0 = 0; n0 < NP; n0 += NC) {
+          if (qvalid) {
 #pragma unroll
-          // exact (|sum| <= 2^24); the conversion pipe is otherwise idle, the ALU pipe is the slicers'
-          for (int j = 0; j < DIGITS; j++) R[j] = rvalid ? __float2int_rn(__uint_as_float(raw[j][x])) : 0;
-          // rotate so that R[t] holds the pair (i0+1, j) of level t+2, i.e. j-1 = t - i0
+            for (int j = 0; j < DIGITS; j++)
 #pragma unroll
-          for (int b = 1; b < DIGITS; b <<= 1) {
-            if (i0 & b) {
-              int T[DIGITS];
+              for (int x = 0; x < NC; x++) D[(j * NC + x) * DSTRIDE + r] = acc[j * NP + n0 + x];
+          }
+          drainers_sync();
+          for (int e = dtid; e < M * min(NC, N - n0); e += NDRAIN * 32) {
+            const int mm = e % M, x = e / M;
+            const int* Dc = D + x * DSTRIDE + mm;
+            long long sv[8];
 #pragma unroll
-              for (int t = 0; t < DIGITS; t++) T[t] = R[(t - b + DIGITS) % DIGITS];
+            for (int t = 0; t < DIGITS; t++) {
+              int sum = 0;  // |sum| <= 8 * MAXSUM * 2^24
 #pragma unroll
-              for (int t = 0; t < DIGITS; t++) R[t] = T[t];
+              for (int i = 0; i <= t; i++) sum += Dc[(t - i) * NC * DSTRIDE + i * MP];
+              sv[t] = sum;
             }
+            const long long vhi = (sv[0] << 24) + (sv[1] << 16) + (sv[2] << 8) + sv[3];
+            const long long vlo = (sv[4] << 24) + (sv[5] << 16) + (sv[6] << 8) + sv[7];
+            const int ea = ae[mm], eb = ae[(p.gram ? 0 : 16) + n0 + x];
+            const double v = fma((double)vlo, 0x1p-32, (double)vhi);  // in units of 2^(EA+EB-2080)
+            double& ca = cacc[(n0 + x) * M + mm];
+            // (one factor where it is in range, so that a small one of the two does not round v)
+            const int es = ea + eb - 2080;
+            ca = (unsigned)(es + 1022) <= 2045u ? fma(v, pow2i(es), ca)
+                                                : fma(v * pow2i(ea - 1040), pow2i(eb - 1040), ca);
           }
-          int c[DIGITS];
+          drainers_sync();
+        }
 #pragma unroll
-          for (int t = 0; t < DIGITS; t++) c[t] = (i0 <= t) ? R[t] : 0;
-          level_reduce(c, MP);
-          if (lane < MP && rvalid && n < N) {
+        for (int x = 0; x < DIGITS * NP; x++) acc[x] = 0;
+        cnt = 0;
+      }
+      if (done) break;
+      if (cnt == 0) {
+        drainers_sync();  // ae has been read
+        if (dtid < 32) ae[dtid] = pe[set * 32 + dtid];
+      }
+      if (qvalid) {
 #pragma unroll
-            for (int t = 0; t < DIGITS; t++) atomicAdd(&S[(t * 16 + m) * 16 + n], c[t]);
-          }
+        for (int b = 0; b < DIGITS * NB; b++) {
+          uint32_t tmp[BN];
+          tmem_ld<BN>(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(set * p.nmma + b * BN), tmp);
+          tmem_wait_ld();
+          // exact (|sum| <= 2^24)
+#pragma unroll
+          for (int x = 0; x < BN; x++) acc[b * BN + x] += __float2int_rn(__uint_as_float(tmp[x]));
         }
       }
+      cnt++;
+      done = last;
       tc_fence_before();
-      drainers_sync();
-      for (int e = dtid; e < M * N; e += NDRAIN * 32) {
-        const int mm = e % M, nn = e / M;
-        long long sv[8];
-#pragma unroll
-        for (int t = 0; t < 8; t++) sv[t] = S[(t * 16 + mm) * 16 + nn];
-        const long long vhi = (sv[0] << 24) + (sv[1] << 16) + (sv[2] << 8) + sv[3];
-        const long long vlo = (sv[4] << 24) + (sv[5] << 16) + (sv[6] << 8) + sv[7];
-        const int ea = pe[set * 32 + mm], eb = pe[set * 32 + (p.gram ? nn : 16 + nn)];
-        const double v = fma((double)vlo, 0x1p-32, (double)vhi);  // in units of 2^(EA+EB-2080)
-        cacc[e] = fma(v * pow2i(ea - 1040), pow2i(eb - 1040), cacc[e]);
-      }
-      drainers_sync();
-      for (int e = dtid; e < SBYTES / 4; e += NDRAIN * 32) S[e] = 0;  // before the next period's atomics
-      if (dtid == 0) mbar_arrive(&drained[set]);
-      if (last) break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&drained[set]);
     }
   } else {
-    // ---- slicers: one unit = one column and 8 rows; A units first, then B units ------------------
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    // ---- slicers: one unit = one column and 8 rows per thread; A units first, then B units -------
     const int NUA = (p.rr / 8) * MP;
-    const int NUB = p.gram ? 0 : (p.rr / 8) * NP;
-    const int NU = NUA + NUB;  // <= 2 * SLICERS (host guarantees)
-    int ucol[2], uoct[2], uop[2];
-    bool uval[2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const int u = tid + k * SLICERS;
-      if (u < NUA) {
-        uop[k] = 0;
-        ucol[k] = u % MP;
-        uoct[k] = u / MP;
-        uval[k] = ucol[k] < M;
-      } else {
-        const int v = u - NUA;
-        uop[k] = 1;
-        ucol[k] = v % NP;
-        uoct[k] = v / NP;
-        uval[k] = u < NU && ucol[k] < N;
-      }
-    }
-    int Ereg[2] = {0, 0};
-    int pp = -1, period_rows = 0;
+    const int NU = NUA + (p.gram ? 0 : (p.rr / 8) * NP);  // <= SLICERS (host guarantees)
+    const bool isB = tid >= NUA;
+    const int uv = isB ? tid - NUA : tid, CP = isB ? NP : MP;
+    const int col = uv % CP, oct = uv / CP;
+    const bool uval = tid < NU && col < (isB ? N : M);
+    const int64_t ld = isB ? p.ldb : p.lda;
+    const TI* gsrc = static_cast<const TI*>(isB ? p.B : p.A);
+    const uint32_t lbo = isB ? p.lbo_b : p.lbo_a;
+    // The 8 rows of an octet o are visited in the order q ^ (o & 7), the same for A and B (a
+    // permutation of k inside a k-octet leaves the MMA's sum unchanged): lanes of a half-warp
+    // holding different octets then read different banks of the FP64 stage.
+    const int g = oct & 7;
+    int Ereg = 0;
+    bool slow = true;  // warp-uniform: a column of this warp may hold subnormal numbers in its range
+    int pp = -1, period_rows = 0, s = -1, d = -1, elast = -1;
+    uint32_t sph = 1, dph = 1;
     for (int t = 0; t < nt; t++) {
-      const int s = t % p.stages, d = t % DST;
+      if (++s == p.stages) s = 0;
+      if (s == 0) sph ^= 1u;
+      if (++d == DST) d = 0;
+      if (d == 0) dph ^= 1u;
       const int64_t tt = t_begin + t;
-      const int64_t r0 = tt * p.rr;
-      const int rows = (int)((p.K - r0) < p.rr ? (p.K - r0) : p.rr);
-      const bool ok = wait_ab(&full[s], (uint32_t)((t / p.stages) & 1), abort_f, p.err);
-      const bool blk = is_bulk(tt);
-      const TI* stA = reinterpret_cast<const TI*>(ring + (size_t)s * p.stage_bytes);
-      const TI* stB = p.gram ? stA : reinterpret_cast<const TI*>(ring + (size_t)s * p.stage_bytes + p.tile_a);
-      double v[2][8];
-      uint32_t eu[2] = {0u, 0u};
-      bool exceed = false;
-      // The 8 rows of an octet o are visited in the order q ^ (o & 7), the same for A and B (a
-      // permutation of k inside a k-octet leaves the MMA's sum unchanged): lanes of a half-warp
-      // holding different octets then read different banks of the FP64 stage.
+      bool ok = mbar_wait_warp(&full[s], sph, abort_f);
+      double v[8];
+      if (is_bulk(tt)) {  // shared-memory stage
+        const TI* src = reinterpret_cast<const TI*>(ring + (size_t)s * p.stage_bytes + (isB ? p.tile_a : 0)) +
+                        (oct * 8) * (int)ld + col;
 #pragma unroll
-      for (int k = 0; k < 2; k++) {
-        const bool isB = uop[k] != 0;
-        const int64_t ld = isB ? p.ldb : p.lda;
-        const int g = uoct[k] & 7;
-        if (blk) {  // shared-memory stage
-          const TI* src = isB ? stB : stA;
-#pragma unroll
-          for (int q2 = 0; q2 < 8; q2++) {
-            const int rr = uoct[k] * 8 + (q2 ^ g);
-            v[k][q2] = (ok && uval[k]) ? (double)src[rr * ld + ucol[k]] : 0.0;
-          }
-        } else {  // global memory (rows not 16-byte aligned, or the last round)
-          const TI* src = static_cast<const TI*>(isB ? p.B : p.A) + r0 * ld;
-#pragma unroll
-          for (int q2 = 0; q2 < 8; q2++) {
-            const int rr = uoct[k] * 8 + (q2 ^ g);
-            v[k][q2] = (ok && uval[k] && rr < rows) ? (double)src[rr * ld + ucol[k]] : 0.0;
-          }
-        }
-        // largest exponent field of the unit (1 if only subnormals, 0 if all zero): the largest
-        // high word without its sign bit gives the field; an OR of the magnitudes tells zero
-        uint32_t hmax = 0u, nz = 0u;
+        for (int q2 = 0; q2 < 8; q2++) v[q2] = uval ? (double)src[(q2 ^ g) * (int)ld] : 0.0;
+      } else {  // global memory (rows not 16-byte aligned, or the last round)
+        const int64_t r0 = tt * p.rr;
+        const int rows = (int)((p.K - r0) < p.rr ? (p.K - r0) : p.rr);
 #pragma unroll
         for (int q2 = 0; q2 < 8; q2++) {
-          const uint32_t h = (uint32_t)__double2hiint(v[k][q2]) & 0x7FFFFFFFu;
-          hmax = max(hmax, h);
-          nz |= h | (uint32_t)__double2loint(v[k][q2]);
+          const int rr = oct * 8 + (q2 ^ g);
+          v[q2] = (uval && rr < rows) ? (double)gsrc[(r0 + rr) * ld + col] : 0.0;
         }
-        eu[k] = hmax >> 20;
-        if (eu[k] == 0u && nz != 0u) eu[k] = 1u;
-        if (uval[k] && (int)eu[k] > Ereg[k]) exceed = true;
       }
+      // largest exponent field of the unit (1 if only subnormals, 0 if all zero): the largest
+      // high word without its sign bit gives the field; an OR of the magnitudes tells zero
+      uint32_t hmax = 0u, nz = 0u;
+#pragma unroll
+      for (int q2 = 0; q2 < 8; q2++) {
+        const uint32_t h = (uint32_t)__double2hiint(v[q2]) & 0x7FFFFFFFu;
+        hmax = max(hmax, h);
+        nz |= h | (uint32_t)__double2loint(v[q2]);
+      }
+      uint32_t eu = hmax >> 20;
+      if (eu == 0u && nz != 0u) eu = 1u;
+      const bool exceed = uval && (int)eu > Ereg;
       const bool newp = pp < 0 || period_rows + p.rr > PERIOD || exceed;
       bool first = false;
       if (slicers_any(!ok || newp)) {
-        if (slicers_any(!ok)) break;
+        if (slicers_any(!ok)) {
+          *abort_f = 1;
+          if (lane == 0) atomicExch(p.err, SKINNY_DEVERR_TIMEOUT);
+          break;
+        }
         // a new period: raise the exponents of the columns that met larger elements
-#pragma unroll
-        for (int k = 0; k < 2; k++)
-          if (uval[k] && (int)eu[k] > Ereg[k]) atomicMax(&Ecur[uop[k] * 16 + ucol[k]], (int)eu[k] + HEAD);
+        if (exceed) atomicMax(&Ecur[(isB ? 16 : 0) + col], (int)eu + HEAD);
         pp++;
         bool ok2 = true;  // the period's exponent slot and accumulator set held period pp - 2
         if (pp >= 2) ok2 = wait_ab(&drained[pp & 1], (uint32_t)(((pp - 2) >> 1) & 1), abort_f, p.err);
         if (slicers_any(!ok2)) break;  // also orders the atomics before the reads below
-        if (tid < 32) pe[(pp & 1) * 32 + tid] = Ecur[tid];
-#pragma unroll
-        for (int k = 0; k < 2; k++) Ereg[k] = uval[k] ? Ecur[uop[k] * 16 + ucol[k]] : 0;
+        if (warp == 0) {
+          const int e = Ecur[lane];
+          pe[(pp & 1) * 32 + lane] = e;
+          const int chg = __any_sync(0xffffffffu, e != elast);
+          if (lane == 0) pchg[pp & 1] = chg;
+          elast = e;
+        }
+        if (uval) Ereg = Ecur[(isB ? 16 : 0) + col];
+        slow = __any_sync(0xffffffffu, uval && Ereg <= EMIN_FAST);
         period_rows = 0;
         first = true;
       }
       // the FP64 stage is consumed: the values are in registers
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
-      int okd = 1;  // the digit stage is free once the MMAs of round t - DST completed
-      if (t >= DST) {
-        if (lane == 0) okd = wait_ab(&dempty[d], (uint32_t)(((t / DST) - 1) & 1), abort_f, p.err);
-        okd = __shfl_sync(0xffffffffu, okd, 0);
-      }
-      if (okd) {
-#pragma unroll
-        for (int k = 0; k < 2; k++)
-          if (uval[k]) {
-            if (uop[k])
-              slice_unit(v[k], (uint32_t)Ereg[k], ucol[k], NP, uoct[k], p.lbo_b, digB(d));
-            else
-              slice_unit(v[k], (uint32_t)Ereg[k], ucol[k], MP, uoct[k], p.lbo_a, digA(d));
-          }
+      // the digit stage is free once the MMAs of round t - DST completed
+      if (t >= DST) ok = mbar_wait_warp(&dempty[d], dph ^ 1u, abort_f);
+      if (__all_sync(0xffffffffu, ok)) {
+        if (uval) {
+          unsigned char* buf = (isB ? digB(d) : digA(d)) + oct * lbo;
+          if (slow)
+            slice_unit<false>(v, (uint32_t)Ereg, col, CP, buf);
+          else
+            slice_unit<true>(v, (uint32_t)Ereg, col, CP, buf);
+        }
         if (tid == 0) rinfo[d] = pp | (first ? (1 << 30) : 0);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&dfull[d]);
+      } else {
+        *abort_f = 1;
+        if (lane == 0) atomicExch(p.err, SKINNY_DEVERR_TIMEOUT);
       }
       period_rows += p.rr;
     }
@@ -575,6 +583,11 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
 
   tc_fence_before();
   __syncthreads();
+  // back to the registers of the launch (a warpgroup's warps have met since the first change)
+  if (warp >= NSLICE && warp < WPROD)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+  else
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(p.tmem_cols));
   if (*abort_f) return;  // timeout recorded in the error word; no partial, no ticket
 
@@ -713,7 +726,7 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   a.MP = a.gram ? NP : pow2ceil(M);
   a.NP = NP;
   // rows per round: 128 * R with R the largest power of two whose slicing units (one column and
-  // 8 rows each) fit two per slicer thread and whose FP64 and digit stages fit in shared memory
+  // 8 rows each) fit one per slicer thread and whose FP64 and digit stages fit in shared memory
   // (at least two of each; bulk copies of whole rounds where aligned dense rows fit, else the
   // slicers read global memory).  A round's fixed costs -- the slicers' barrier, the hand-offs,
   // the MMA commit -- then spread over as many rows as possible.
@@ -729,7 +742,7 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   int64_t dstage = 0;
   a.stages = 0;
   for (int R = PERIOD / 128; R >= 1 && a.stages == 0; R /= 2) {
-    if (R * 16 * cols > 2 * SLICERS) continue;
+    if (R * 16 * cols > SLICERS) continue;
     a.rr = 128 * R;
     const int64_t octs = a.rr / 8;
     a.dig_a = (uint32_t)round_up(octs * a.lbo_a + DPAD, 1024);

@@ -153,7 +153,8 @@ __device__ __forceinline__ uint32_t exp_field(double x) {
 // 8 balanced digits of x relative to exponent field E (most significant first), as exact floats
 __device__ __forceinline__ void digits_of(double x, uint32_t E, float (&d)[DIGITS], bool& neg) {
   uint32_t gh, gl;
-  g_words(x, E, gh, gl, neg);
+  g_words(x, E, gh, gl);
+  neg = (__double2hiint(x) >> 31) != 0;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     d[i] = __uint_as_float(0x4B000000u | ((gh >> (8 * (3 - i))) & 0xFF)) - 8388736.0f;
@@ -508,11 +509,11 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
         uint32_t dp[4][DIGITS];  // element pairs (0,1), (2,3), (4,5), (6,7) of the octet
 #pragma unroll
         for (int q2 = 0; q2 < 4; q2++) {
+          const double a = v[o * 8 + 2 * q2], b = v[o * 8 + 2 * q2 + 1];
           uint32_t gha, gla, ghb, glb;
-          bool na, nb;
-          g_words(v[o * 8 + 2 * q2], emax, gha, gla, na);
-          g_words(v[o * 8 + 2 * q2 + 1], emax, ghb, glb, nb);
-          digit_pairs(gha, gla, na, ghb, glb, nb, dp[q2]);
+          g_words(a, emax, gha, gla);
+          g_words(b, emax, ghb, glb);
+          digit_pairs(gha, gla, ghb, glb, sign_pair(a, b), dp[q2]);
         }
         // plane pl holds digit pl + 1: 128 rows x MP columns, k-octets 2048 bytes apart
 #pragma unroll

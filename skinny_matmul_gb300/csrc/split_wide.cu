@@ -180,22 +180,6 @@ __device__ __forceinline__ bool wait_ab(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
-// the same for the slicers, all lanes of a warp at once and without a branch where the phase is
-// complete already (a wait by one lane of a warp, with a warp barrier, cost ~150 clocks more); false: it ran out
-__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile int* ab) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p, q;\n .reg .b32 i, a;\n mov.b32 i, 0;\n"
-      "W_%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n @p bra D_%=;\n"
-      " ld.volatile.shared.b32 a, [%3];\n add.u32 i, i, 1;\n"
-      " setp.lt.u32 q, i, 4194304;\n setp.eq.and.b32 q, a, 0, q;\n @q bra W_%=;\n"
-      "D_%=:\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<int*>(ab)))
-      : "memory");
-  return ok != 0;
-}
-
 // signed fixed-point value of x relative to exponent field E, offset for balanced base-256 digits
 __device__ __forceinline__ uint64_t fixed_g(double x, uint32_t E) {
   const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
@@ -605,7 +589,7 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
       if (rs == 0) rph ^= 1u;
       if (++ds == DSLOTS) ds = 0;
       if (ds == 0) dph ^= 1u;
-      ok &= wait_warp(&raw_full[rs], rph, abort_f);
+      ok &= mbar_wait_warp(&raw_full[rs], rph, abort_f);
       const int rows = (int)min((int64_t)SR, p.K - (s_begin + ls) * SR);
       const TI* T = reinterpret_cast<const TI*>(raw + (size_t)rs * p.raw_stage) + tofs;
       auto get = [&](int k) {
@@ -670,7 +654,7 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
         vflag[ls & 3] = ls + 1;
         slow = __any_sync(0xffffffffu, Ecur <= EMIN || (F32 && Ecur > EOFS + 254 && cvalid));
       }
-      if (ls >= DSLOTS) ok &= wait_warp(&dempty[ds], dph ^ 1u, abort_f);
+      if (ls >= DSLOTS) ok &= mbar_wait_warp(&dempty[ds], dph ^ 1u, abort_f);
       // slice: digits relative to Ecur into slot ds
       unsigned char* sa = dig + (size_t)ds * SLOT;
       unsigned char* sb = sa + SLOT_A;
