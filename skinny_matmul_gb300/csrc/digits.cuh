@@ -62,13 +62,4 @@ __device__ __forceinline__ void digit_pairs2(uint32_t ga, uint32_t gb, int lower
   d1 = dig(0x4342);
 }
 
-// the eight digit pairs, digit i in out[i]
-__device__ __forceinline__ void digit_pairs(uint32_t gha, uint32_t gla, uint32_t ghb, uint32_t glb, SignPair sg,
-                                            uint32_t (&out)[NDIGITS]) {
-  digit_pairs2(gha, ghb, 0, sg, out[0], out[1]);
-  digit_pairs2(gha, ghb, 1, sg, out[2], out[3]);
-  digit_pairs2(gla, glb, 0, sg, out[4], out[5]);
-  digit_pairs2(gla, glb, 1, sg, out[6], out[7]);
-}
-
 }  // namespace skinny

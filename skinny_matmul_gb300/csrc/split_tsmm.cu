@@ -9,7 +9,7 @@
 //     shared exponent f_n; row r of A gets the exponent e_r of its largest element.  Every value
 //     becomes a 62-bit fixed-point integer and 8 balanced base-256 digits (exact in FP16), as in
 //     the split TSMTTSM (split.cu); A's digits are formed with byte permutes and one HFMA2 per
-//     digit pair (digit_pairs).
+//     digit pair (digit_pairs2).
 //   * Digit-stacked MMAs: for A digit i, one tcgen05.mma (M = 128 rows, K = 16 columns m) against
 //     B's digit planes j = 1..9-i stacked along N gives every pair (i, j) with i + j <= 9 at once,
 //     written to the accumulator columns of level L = i + j (level L at columns (L-2) NB of a block
@@ -18,8 +18,8 @@
 //     leading level).  |D_L| <= 2^14 MP (L - 2) (the top digit is at most 64 in magnitude): exact
 //     in the FP32 TMEM accumulators.
 //   * Epilogue: V = sum_L D_L 2^(8(9-L)) (|V| < 2^74) is formed as a 64-bit integer W = V / 2^12
-//     (level_window), rounded to a double (by integer instructions or the FP64 pipe's conversion) and scaled by 2^(e_r + f_n - 2100) in the exponent field; beta*C
-//     is one FMA.
+//     (level_window), rounded to a double (by integer instructions or the FP64 pipe's conversion)
+//     and scaled by 2^(e_r + f_n - 2100) in the exponent field; beta*C is one FMA.
 //   * Warp roles, hand-offs through mbarriers, no CTA-wide barrier while streaming (16 or 24 warps):
 //       slicers     (8 warps, two threads per row) read the FP64 values of a 128-row tile (the
 //                   next tile's are loaded right after a tile is sliced), take the row exponent,
@@ -43,6 +43,7 @@
 #include <cuda_fp16.h>
 
 #include <cstring>
+#include <type_traits>
 
 #include "api_internal.h"
 #include "digits.cuh"
@@ -318,6 +319,13 @@ __device__ __forceinline__ bool wait_ab(uint64_t* bar, uint32_t parity, volatile
   if (err) atomicExch(err, SKINNY_DEVERR_TIMEOUT);
   return false;
 }
+// the same without sleeping, by all lanes of a warp (8 x 32 with beta, 0.8 GiB of A: 614 -> 572 us)
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile int* ab, int* err) {
+  if (mbar_wait_warp(bar, parity, ab)) return true;
+  *ab = 1;
+  if (err) atomicExch(err, SKINNY_DEVERR_TIMEOUT);
+  return false;
+}
 // asynchronous global -> shared copies of old C (src_bytes < size zero-fills the rest; 0 reads nothing)
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
@@ -491,9 +499,10 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
       for (int j = 0; j < PART; j++) emax = max(emax, exp_field(v[j]));
 #pragma unroll
       for (int o = 1; o < TPS; o *= 2) emax = max(emax, (uint32_t)__shfl_xor_sync(0xffffffffu, emax, o));
+      const bool fast = __all_sync(0xffffffffu, emax > EMIN_FAST);
       bool ok = *abort_f == 0;
-      if (ok && it >= RE) ok = wait_ab(&eempty[es], eph, abort_f, p.err);
-      if (ok && it >= p.nast) ok = wait_ab(&aempty[s], sph, abort_f, p.err);
+      if (ok && it >= RE) ok = wait_warp(&eempty[es], eph, abort_f, p.err);
+      if (ok && it >= p.nast) ok = wait_warp(&aempty[s], sph, abort_f, p.err);
       if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp leaves together
       if (part == 0) erow[es * ROWS + row] = (int)emax;
       unsigned char* A_ = adig + (size_t)s * p.astage;
@@ -506,20 +515,31 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
             *reinterpret_cast<uint4*>(A_ + (uint32_t)(pl * MP * 256) + kmaj(row, mo, 2048u)) = make_uint4(0, 0, 0, 0);
           continue;
         }
-        uint32_t dp[4][DIGITS];  // element pairs (0,1), (2,3), (4,5), (6,7) of the octet
+        // plane pl holds digit pl + 1: 128 rows x MP columns, k-octets 2048 bytes apart.  fast: rows whose
+        // largest element leaves no subnormal number in range (16 x 16, 0.5 GiB: 520 -> 489 us with
+        // beta, 450 -> 440 without, together with the shorter waits)
+        auto slice = [&](auto fast) {
+          uint32_t gw[2][8];
+          SignPair sg[4];
 #pragma unroll
-        for (int q2 = 0; q2 < 4; q2++) {
-          const double a = v[o * 8 + 2 * q2], b = v[o * 8 + 2 * q2 + 1];
-          uint32_t gha, gla, ghb, glb;
-          g_words(a, emax, gha, gla);
-          g_words(b, emax, ghb, glb);
-          digit_pairs(gha, gla, ghb, glb, sign_pair(a, b), dp[q2]);
-        }
-        // plane pl holds digit pl + 1: 128 rows x MP columns, k-octets 2048 bytes apart
+          for (int k = 0; k < 8; k++) g_words<decltype(fast)::value>(v[o * 8 + k], emax, gw[0][k], gw[1][k]);
 #pragma unroll
-        for (int pl = 0; pl < DIGITS; pl++)
-          *reinterpret_cast<uint4*>(A_ + (uint32_t)(pl * MP * 256) + kmaj(row, mo, 2048u)) =
-              make_uint4(dp[0][pl], dp[1][pl], dp[2][pl], dp[3][pl]);
+          for (int q2 = 0; q2 < 4; q2++) sg[q2] = sign_pair(v[o * 8 + 2 * q2], v[o * 8 + 2 * q2 + 1]);
+          unsigned char* dst = A_ + kmaj(row, mo, 2048u);
+#pragma unroll
+          for (int pl = 0; pl < DIGITS; pl += 2) {
+            uint32_t d0[4], d1[4];
+#pragma unroll
+            for (int q2 = 0; q2 < 4; q2++)
+              digit_pairs2(gw[pl / 4][2 * q2], gw[pl / 4][2 * q2 + 1], pl & 2, sg[q2], d0[q2], d1[q2]);
+            *reinterpret_cast<uint4*>(dst + pl * MP * 256) = make_uint4(d0[0], d0[1], d0[2], d0[3]);
+            *reinterpret_cast<uint4*>(dst + (pl + 1) * MP * 256) = make_uint4(d1[0], d1[1], d1[2], d1[3]);
+          }
+        };
+        if (MP <= 32 && fast)  // (at 64 the second copy of the code costs more than it saves: 439 us, 431 without)
+          slice(std::true_type{});
+        else
+          slice(std::false_type{});
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -610,7 +630,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
       if (issuer && it + p.la < nt) issue_tile();  // a timeout sets the abort flag
       const int64_t rr = row0 + it * rstep + r;
       const bool live = rr < p.K;
-      ok = wait_ab(&efull[es], eph, abort_f, p.err);
+      ok = wait_warp(&efull[es], eph, abort_f, p.err);
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -625,7 +645,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
       T* crow = static_cast<T*>(p.C) + rr * p.ldc;
       int c = eg;  // this warp's chunks are c = eg (mod EG)
       for (int cb = 0; cb < p.ncb; cb++) {
-        ok = wait_ab(&tfull[k], kp, abort_f, p.err);
+        ok = wait_warp(&tfull[k], kp, abort_f, p.err);
         if (!__all_sync(0xffffffffu, ok)) {
           ok = false;
           break;
