@@ -41,9 +41,13 @@ __device__ __forceinline__ void g_words(double x, uint32_t E, uint32_t& gh, uint
 struct SignPair {
   uint32_t s, c;
 };
-__device__ __forceinline__ SignPair sign_pair(double a, double b) {
-  const uint32_t t = __byte_perm((uint32_t)__double2hiint(a), (uint32_t)__double2hiint(b), 0x7632) & 0x80008000u;
+// (from the words that hold their sign bits)
+__device__ __forceinline__ SignPair sign_pair(uint32_t a, uint32_t b) {
+  const uint32_t t = __byte_perm(a, b, 0x7632) & 0x80008000u;
   return {t | 0x3C003C00u, t ^ 0xE480E480u};
+}
+__device__ __forceinline__ SignPair sign_pair(double a, double b) {
+  return sign_pair((uint32_t)__double2hiint(a), (uint32_t)__double2hiint(b));
 }
 // Two FP16 digit pairs of elements a, b (a in the low halves) from one 32-bit word of their G's: the
 // digits of its upper (half 0) or lower bytes, the higher one in d0.  A byte g of G becomes the half

@@ -10,8 +10,8 @@
 // Scheme:
 //   * Per column of A (and of B) a shared exponent E holds for an epoch: an element x is
 //     x = sign * F * 2^(E - 1084) with F < 2^62 a fixed-point integer, and F is written as 8
-//     balanced base-256 digits d_1..d_8 (d_1 in [-64, 64], the others in [-128, 127]).  The
-//     sign is applied to F before splitting, so the digits of a negative x are the digits of -F.
+//     balanced base-256 digits d_1..d_8 (d_1 in [-64, 64], the others in [-128, 127]), to each of
+//     which the sign of x is applied (digits.cuh).
 //     When a column meets an element larger than 2^E allows, E is raised (with 4 bits of
 //     headroom) and a new epoch starts for the whole CTA (drained words do not mix exponents).
 //   * Digits are exact in FP16.  For a stage of 16 rows the digits are laid out as FP16 planes
@@ -19,14 +19,17 @@
 //     [0, 1, 5 | 0, 2, 6 | 0, 3, 7 | 0, 4, 8] (0 = a zero plane, p = digit p of the 64 columns),
 //     so the 128-row window [A_i ; A_{i+4}] is contiguous for i = -3..4; B' holds the planes
 //     [0, 1, 2, ..., 8], so the 128-row window [B_j ; B_{j+1}] is contiguous for j = 0..7.
-//   * One tcgen05.mma (M = N = 128, K = 16, FP16 x FP16 -> FP32 in TMEM) of window i of A' and
-//     window j of B' forms four 64 x 64 quadrants at digit levels (i + j, i + j + 1) in TMEM
-//     lanes 0..63 and (i + j + 4, i + j + 5) in lanes 64..127.  Two accumulators
+//   * A tcgen05.mma (M = 128, K = 16, FP16 x FP16 -> FP32 in TMEM) of window i of A' and
+//     planes j, j + 1 of B' forms four 64 x 64 quadrants at digit levels (i + j, i + j + 1) in TMEM
+//     lanes 0..63 and (i + j + 4, i + j + 5) in lanes 64..127.  Two accumulators of 128 columns
 //     collect all 36 digit pairs with level i + j <= 9:
 //        key 2:  i = -3..2, j = 2 - i   -> levels 2, 3 (lanes 0-63) and 6, 7 (lanes 64-127)
 //        key 4:  i = -3..4, j = 4 - i   -> levels 4, 5 and 8, 9
-//     14 MMAs per 16 rows; each pair is counted once.  Levels >= 10 are dropped (weight below
-//     2^-56 of the leading level).
+//     For i <= 2 the two keys' planes 2 - i .. 5 - i are adjacent, so one MMA with N = 256 serves
+//     both and reads the window of A' once: 8 MMAs per 16 rows (14 with N = 128, each with its own
+//     read of both operands, 12 KB against 16 per window: 64 x 64, K = 2^20, 428 -> 415 us; the
+//     operand reads, not the products, bound them).  Each pair is counted once.  Levels >= 10
+//     are dropped (weight below 2^-56 of the leading level).
 //   * A cell of an accumulator sums at most 8 digit products per row (|d d| <= 2^14), so over a
 //     period of 128 rows every partial sum is an integer of magnitude < 2^24 and the FP32
 //     accumulation is exact.  The two accumulators take 256 TMEM columns; two sets alternate
@@ -43,13 +46,13 @@
 //     warp, which raises its exponent by itself, leaves (stage, exponent before, since) for the drain
 //     warps and marks the stage for the MMA warp.  Every wait is bounded; a wait that runs
 //     out sets the error word and the CTA finishes without waiting further and writes no C.
-//   * Bound: a stage of 16 x (64 + 64) values takes ~1800 clocks, in which the schedulers issue in 67 %
-//     (slicing: ~28 instructions a value), the tensor pipe is busy in 900 (14 MMAs of 64) and a TMA
-//     copy of the same rows would take ~700.  With 8 warps that sliced and drained by turns and voted
+//   * Bound: a stage of 16 x (64 + 64) values takes ~1650 clocks.  The MMAs alone take ~1400 (900 of
+//     products; operands from shared memory), slicing alone ~1400 (~25 instructions a value, two
+//     thirds of the issue slots), and a TMA copy of the same rows would take ~700.  With 8 warps that sliced and drained by turns and voted
 //     on the exponents of each stage it was 3600: each step of a stage (two mbarriers, the vote, the
-//     drain) was waited out by all of them.  Measured, K rows: f64 64 x 64, K = 2^20, 794 -> 431 us;
-//     32 x 32, K = 2^22, 1252 -> 745; 48 x 24, K = 2^20, 714 -> 358; Gram 64, K = 2^20, 738 -> 403;
-//     rows of 80 (64 x 64, K = 2^20) 776 -> 616; f32 64 x 64, K = 2^18, 308 -> 156.
+//     drain) was waited out by all of them.  Measured, K rows: f64 64 x 64, K = 2^20, 794 -> 395 us;
+//     32 x 32, K = 2^22, 1252 -> 680; 48 x 24, K = 2^20, 714 -> 325; Gram 64, K = 2^20, 738 -> 367;
+//     rows of 80 (64 x 64, K = 2^20) 776 -> 586; f32 64 x 64, K = 2^18, 308 -> 149.
 //   * Blocks of 64 x 64 (M or N > 64) run in the same launch, as do the row chunks of every
 //     block; the last CTA of a block (ticket) sums the chunks' partials in chunk order and
 //     applies alpha and beta.  Gram (A = B) computes the upper blocks only and mirrors them.
@@ -59,12 +62,11 @@
 //     (the off-diagonal quadrants pair different rows and are not read), so a 32-wide product
 //     uses every slicer and every MMA column, and the halves are added at the end.
 // Inputs must be finite (Inf/NaN have no fixed-point form).
-#include <cuda_fp16.h>
-
 #include <atomic>
 #include <cstring>
 
 #include "api_internal.h"
+#include "digits.cuh"
 
 namespace skinny {
 
@@ -127,11 +129,13 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n selp.u32 %0, 1, 0, e;\n}\n" : "=r"(p));
   return p != 0;
 }
-__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+// (descriptors as their lower words: the upper ones are constants)
+__device__ __forceinline__ void mma_f16(uint32_t tmem, uint32_t da, uint32_t db, uint32_t idesc, uint32_t acc) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-      "l"(da), "l"(db), "r"(idesc), "r"(acc));
+      "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n"
+      " mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem),
+      "r"(da), "r"(db), "r"(idesc), "r"(acc), "n"((128 >> 4) | (1 << 14)));
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -180,20 +184,9 @@ __device__ __forceinline__ bool wait_ab(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
-// signed fixed-point value of x relative to exponent field E, offset for balanced base-256 digits
-__device__ __forceinline__ uint64_t fixed_g(double x, uint32_t E) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t ef = (hi >> 20) & 0x7FF;
-  const uint32_t eff = ef ? ef : 1u;
-  const uint64_t mant = ((uint64_t)((hi & 0xFFFFFu) | (ef ? 0x100000u : 0u)) << 32) | lo;
-  const uint32_t sh = E - eff;  // E >= eff for every nonzero element of the epoch
-  uint64_t F = sh < 64 ? ((mant << 9) >> sh) : 0ull;
-  if (hi >> 31) F = 0ull - F;
-  return F + 0x8080808080808080ull;
-}
-
-// the same for E > 64 (FP32: E > 64 above its exponents' offset), where zeros and subnormal numbers
-// shift out entirely and need no case of their own; sh = E - exponent field >= 0
+// G (digits.cuh) of an element from its bits (FP32: hi) and sh = E - exponent field >= 0, for E > 64
+// (FP32: 64 above the offset of its exponents), where zeros and subnormal numbers shift out entirely
+// and need no case of their own
 template <typename TI>
 __device__ __forceinline__ uint64_t fixed_fast(uint32_t hi, uint32_t lo, uint32_t sh) {
   uint32_t H, L;
@@ -206,24 +199,13 @@ __device__ __forceinline__ uint64_t fixed_fast(uint32_t hi, uint32_t lo, uint32_
   }
   uint64_t F;
   asm("shr.u64 %0, %1, %2;" : "=l"(F) : "l"(((uint64_t)H << 32) | L), "r"(sh));  // 0 from 64 on
-  const int64_t sg = (int32_t)hi >> 31;
-  return (F ^ (uint64_t)sg) - (uint64_t)sg + 0x8080808080808080ull;
+  return F + 0x8080808080808080ull;
 }
 // exponent field of x's magnitude (subnormal numbers: 1), 0 for zero; of the FP64 value for FP32
 __device__ __forceinline__ uint32_t exp_field(double x) {
   const uint32_t mh = (uint32_t)__double2hiint(x) & 0x7FFFFFFFu;
   const uint32_t e = mh >> 20;
   return e == 0 && (mh | (uint32_t)__double2loint(x)) ? 1u : e;
-}
-
-// FP16 pair (digit of x, digit of y) from the word (byte_x, 0x64, byte_y, 0x64): value 1024 + g
-// minus 1152 = g - 128, exact.  t interleaves one 32-bit half of the offset fixed-point values of
-// two elements: __byte_perm(x, y, 0x7362) = (x.b2, y.b2, x.b3, y.b3) feeds selectors 0x4342
-// (byte 3: the higher digit) and 0x4140 (byte 2); 0x5140 gives bytes 1 and 0 the same way.
-__device__ __forceinline__ uint32_t half_pair(uint32_t t, uint32_t sel) {
-  uint32_t w = __byte_perm(t, 0x64646464u, sel), d;
-  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(w), "r"(0x64806480u));
-  return d;
 }
 
 __device__ __forceinline__ double pow2i(int e) {  // 2^e, clamped to the normal range
@@ -437,14 +419,16 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
         tc_after();
         const uint32_t a0 = smem_u32(dig) + ds * SLOT;
         if (elect_one()) {
-          const uint64_t da = desc(a0, LBO_A), db = desc(a0 + SLOT_A, LBO_B);  // planes are 1024 bytes apart
+          const uint32_t da = (uint32_t)desc(a0, LBO_A), db = (uint32_t)desc(a0 + SLOT_A, LBO_B);  // planes are 1024 bytes apart
           const uint32_t d0 = tmem + ((periods - 1) & 1) * 256;
   #pragma unroll
-          for (int i = -3; i <= 2; i++)
-            mma_f16(d0, da + 64 * slot_a(i), db + 64 * (2 - i), idesc, i == -3 ? !start : 1u);
-  #pragma unroll
-          for (int i = -3; i <= 4; i++)
-            mma_f16(d0 + 128, da + 64 * slot_a(i), db + 64 * (4 - i), idesc, i == -3 ? !start : 1u);
+          for (int i = -3; i <= 4; i++) {
+            const uint32_t ai = da + 64 * slot_a(i);
+            if (i <= 2)  // both keys: planes 2 - i .. 5 - i
+              mma_f16(d0, ai, db + 64 * (2 - i), idesc + (16u << 17), i == -3 ? !start : 1u);
+            else
+              mma_f16(d0 + 128, ai, db + 64 * (4 - i), idesc, 1u);
+          }
           mma_commit(&dempty[ds]);
         }
         __syncwarp();
@@ -666,17 +650,22 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
             g[k] = fixed_fast<TI>(cur.hi[k], cur.lo[k], Ecur - EOFS - field(cur, k));
         } else {
 #pragma unroll
-          for (int k = 0; k < NR; k++) g[k] = fixed_g(value(cur, k), Ecur);
+          for (int k = 0; k < NR; k++) {
+            uint32_t gh, gl;
+            g_words(value(cur, k), Ecur, gh, gl);
+            g[k] = ((uint64_t)gh << 32) | gl;
+          }
         }
-        // digits d = 2 gi + 1 and d + 1 of each element pair come from one byte interleave
+        SignPair sg[NR / 2];
+#pragma unroll
+        for (int pp = 0; pp < NR / 2; pp++) sg[pp] = sign_pair(cur.hi[2 * pp], cur.hi[2 * pp + 1]);
+        // digits d = 2 gi + 1 and d + 1 of each element pair
         auto digits = [&](int gi, uint32_t (&w1)[NR / 2], uint32_t (&w2)[NR / 2]) {
 #pragma unroll
           for (int pp = 0; pp < NR / 2; pp++) {
             const uint32_t x = gi < 2 ? (uint32_t)(g[2 * pp] >> 32) : (uint32_t)g[2 * pp];
             const uint32_t y = gi < 2 ? (uint32_t)(g[2 * pp + 1] >> 32) : (uint32_t)g[2 * pp + 1];
-            const uint32_t t = __byte_perm(x, y, (gi & 1) ? 0x5140 : 0x7362);
-            w1[pp] = half_pair(t, 0x4342);
-            w2[pp] = half_pair(t, 0x4140);
+            digit_pairs2(x, y, gi & 1, sg[pp], w1[pp], w2[pp]);
           }
         };
         if (GR == 1 || (GR == 2 && gram)) {
