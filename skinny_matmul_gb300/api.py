@@ -17,12 +17,17 @@ from . import lib as L
 _ACC = {"native": L.ACC_NATIVE, "dd": L.ACC_DD, "split": L.ACC_SPLIT, "auto": L.ACC_AUTO}
 
 
+_codes: dict = {}  # torch dtype -> code, filled at the first use (torch is imported late)
+
+
 def _dtype_code(t) -> int:
-    import torch
-    m = {torch.float32: L.R32, torch.float64: L.R64, torch.complex64: L.C32, torch.complex128: L.C64}
-    if t.dtype not in m:
+    if not _codes:
+        import torch
+        _codes.update({torch.float32: L.R32, torch.float64: L.R64, torch.complex64: L.C32, torch.complex128: L.C64})
+    code = _codes.get(t.dtype)
+    if code is None:
         raise TypeError(f"unsupported dtype {t.dtype}")
-    return m[t.dtype]
+    return code
 
 
 def _scalar(v, code):
@@ -42,10 +47,25 @@ def _ptr(x):
     return x.data_ptr()
 
 
+_torch = None  # torch, once imported
+
+
+def _current_stream() -> int:
+    """The current stream's handle.  A short product is bound by the host: the raw query takes 0.4 us,
+    current_stream(), which builds a Stream object, 2.9 (4 x 4 products of 4096 rows, a call: 8.2 us
+    against 10.1, which includes the look-up of the dtype in a dict built once)."""
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    if _torch.cuda.is_initialized():
+        return _torch._C._cuda_getCurrentRawStream(_torch._C._cuda_getDevice())
+    return _torch.cuda.current_stream().cuda_stream
+
+
 def _stream(stream):
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
