@@ -278,21 +278,7 @@ __device__ __forceinline__ long long level_window(const uint32_t (&raw)[8][W], i
   }
   return ((long long)P1 << 36) + (long long)P2 * (1 << 20) + (long long)P3 * 16 + (long long)(P4 >> 12);
 }
-// Integer finisher, ex = er + fc - 1014 (the biased exponent field of the result when W has its
-// leading one at bit 63): normalise |W| so that its leading one is bit 63, round on bit 10 (ties
-// away from zero), and add the exponent field below the leading one, so that a mantissa carry
-// raises the exponent.
-__device__ __forceinline__ double window_int(long long W, int ex) {
-  const uint32_t sgn = (uint32_t)((unsigned long long)W >> 32) & 0x80000000u;
-  const unsigned long long m = (unsigned long long)(W < 0 ? -W : W);
-  const int z = __clzll((long long)m);                       // 64 for W == 0
-  const unsigned long long n = m << (z & 63);                 // leading one at bit 63 (0 for W == 0)
-  const unsigned long long r = (n >> 11) + ((n >> 10) & 1);  // 53 bits, or 2^53 after a carry
-  const int ef = ex - z;                                      // biased exponent field of the result
-  const uint32_t hi = ((uint32_t)(ef - 1) << 20) + (uint32_t)(r >> 32);
-  const bool ok = n != 0 && ef > 0;
-  return __hiloint2double(ok ? (int)(hi | sgn) : 0, ok ? (int)(uint32_t)r : 0);
-}
+// Integer finisher: window_int (digits.cuh) with ex = er + fc - 1014.
 // Conversion finisher, es = er + fc - 2100: the FP64 pipe's int64 -> double conversion (rounded
 // to nearest; exact scaling follows), then es added to the exponent field.
 __device__ __forceinline__ double window_cvt(long long W, int es) {

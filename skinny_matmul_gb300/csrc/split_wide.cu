@@ -481,14 +481,15 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
       const bool last = !ok || *nperiods == idx;
       const int ep = last ? -2 : mepoch[buf];
       if (ep != acc_epoch) {  // warp-uniform: the words so far are complete
-        // (one multiplication where the power of two is in range: the FP64 pipe does 1.89 a clock)
+        // (by integer instructions unless the result could leave the normal range: a conversion and a
+        // multiplication of every cell on the FP64 pipe took 7.2 us at 32 x 32, 12.5 at 64 x 64)
         if (live && (acc_epoch >= 0 || last)) {
 #pragma unroll
           for (int x = 0; x < 32; x++) {
             const int ebx = __shfl_sync(0xffffffffu, eb, x) - 1040 - (hm ? 32 : 0), es = ea - 1040 + ebx;
             if (mv < Mb && x < nlim) {
-              double v = (double)acc[x];
-              v = (unsigned)(es + 1022) <= 2045u ? v * pow2i(es) : v * pow2i(ea - 1040) * pow2i(ebx);
+              const double v = (unsigned)(es + 1022) <= 1980u ? window_int(acc[x], es + 1086)
+                                                              : (double)acc[x] * pow2i(ea - 1040) * pow2i(ebx);
               part[x * 64] = flushed ? part[x * 64] + v : v;
             }
             acc[x] = 0;
@@ -747,7 +748,8 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
     for (int i = 0; i < GROUP; i++) v[i] = i < gsize ? __ldcg(P + (size_t)(grp * GROUP + i) * 8192 + cell) : 0.0;
     double sum = 0.0;
 #pragma unroll
-    for (int i = 0; i < GROUP; i++) sum += v[i];
+    for (int i = 0; i < GROUP; i++)
+      if (i < gsize) sum += v[i];
     G[(size_t)grp * 4096 + cell] = sum;
   }
   __threadfence();
@@ -766,7 +768,8 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
     for (int i = 0; i < 15; i++) v[i] = i < ngroups ? __ldcg(G + (size_t)i * 4096 + cell) : 0.0;
     double sum = 0.0;
 #pragma unroll
-    for (int i = 0; i < 15; i++) sum += v[i];
+    for (int i = 0; i < 15; i++)
+      if (i < ngroups) sum += v[i];
     const int64_t ci = (int64_t)(W * bj + nn) * p.ldc + W * bi + mm;
     const int64_t cmi = (int64_t)(W * bi + mm) * p.ldc + W * bj + nn;
     const bool mirror = p.sym && bi < bj;  // Gram: the mirrored block holds the same sums
