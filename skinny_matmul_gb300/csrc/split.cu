@@ -678,22 +678,24 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
     set_error("split precision TSMTTSM: M, N <= 128");
     return SKINNY_UNSUPPORTED;
   }
-  // auto selection (measured on GB300): the split kernel wins from M*N >= 256 on, and whenever
-  // both widths are at least 8 (8x8 1.07x at 512 MB of operands and 1.29x at K = 2^20, 8x16 1.37x,
-  // 16x8 1.44x; complex 4x8 and 8x4 through the real product 1.3x); below that the CUDA-core FP64
-  // kernel is as fast or faster (4x16 0.71x, 4x32 0.44x).  The wide kernel costs about as much per 64 x 64
-  // block whatever the block's fill (12.5 ms per block at K = 2^24; CUDA-core FP64 takes 23 ms at
-  // M = N = 17 and 114 ms at 64), so it is chosen from M*N >= 320 per block on; with M, N <= 32 its
-  // folded stages halve that cost, and with both widths >= 8 it wins from the smallest such
-  // product on (1 GiB of operands: 17x8 1.9x, 20x8 1.9x, 17x17 4.8x, 32x8 1.8x; 32x4 is a tie and
-  // takes the CUDA-core kernel through the rule above).  The autotuner can override per shape.
+  // auto selection (measured on GB300, us, CUDA-core FP64 kernel / this one):
+  //   * both widths at least 4 and M N >= 32.  Rows of 2^20: 4x8 71/56, 6x6 75/60, 8x8 120/64, 4x16
+  //     128/94, 4x32 244/179, 4x64 489/306; but 4x4 41/40, 16x2 73/87, 2x64 290/308.
+  //   * K M N >= 2^22, or 3 * 2^22 with a width below 8: the kernels' fixed costs differ by 5 to 10 us.  At
+  //     2^22: 8x8 17.2/15.3, 16x16 20.5/16.5, 32x8 21.8/19.1, 32x32 27.7/28.4; at 2^21 12.4/13.4, 15.9/16.4,
+  //     16.5/18.1 and (24x24) 24.2/22.4.  4x16 at 2^22 17.9/18.8, 4x32 at 2^23 27.1/28.3.
+  //   * the wide kernel's blocks of 64 x 64 filled by a quarter of a 32 x 32 or 4 x 64 at least (128
+  //     cells where the stages fold, else 256 a block).
+  // The autotuner can override per shape.
   const bool wide = M > 16 || N > 16;
   const int64_t sym_w = (A == B && lda == ldb && M == N) ? 1 : 0;
   const int64_t bm = (M + 63) / 64, bn = (N + 63) / 64;
   const int64_t nblk_w = sym_w ? bm * (bm + 1) / 2 : bm * bn;
-  const int64_t per_blk = (M <= 32 && N <= 32) ? 128 : 320;
-  const bool narrow_wins = M * N >= 256 || (M >= 8 && N >= 8);
-  if (autoselect && (K < 4096 || !narrow_wins || (wide && M * N < per_blk * nblk_w))) {
+  const int64_t per_blk = (M <= 32 && N <= 32) ? 128 : 256;
+  const bool widths_win = M >= 4 && N >= 4 && M * N >= 32;
+  const int64_t work_min = (M >= 8 && N >= 8) ? (int64_t)1 << 22 : (int64_t)3 << 22;
+  if (autoselect &&
+      (K < 4096 || K * M * N < work_min || !widths_win || (wide && M * N < per_blk * nblk_w))) {
     set_error("split precision: not selected automatically for this shape");
     return SKINNY_UNSUPPORTED;
   }
