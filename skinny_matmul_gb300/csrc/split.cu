@@ -71,9 +71,12 @@ constexpr int MAXST = 4;       // FP64 stages (at most)
 constexpr int MAXDST = 3;      // digit stages (at most)
 constexpr int DPAD = 128 * 16; // slack after an A digit buffer: the MMA reads 128 rows per k-octet
 constexpr int HDR = 2048;      // barriers, TMEM slot, round and period records, exponents
-constexpr int NCMAX = 4;                 // columns of B whose digit pairs the drain sorts by level at a time
-constexpr int DSTRIDE = 128 + 8;
-constexpr int SBYTES = DIGITS * NCMAX * DSTRIDE * 4;
+// columns of B whose digit pairs the drain sorts by level at a time, and the stride of their rows: 4
+// where that leaves the stages as they are, else 2 (8 x 8 at 2^14 rows 14.6 us and 16.4)
+template <int NCB>
+struct SortBuf {
+  static constexpr int NC = NCB, STRIDE = NCB == 4 ? 128 + 8 : 128, BYTES = DIGITS * NCB * STRIDE * 4;
+};
 constexpr int CBYTES = 256 * 8;          // FP64 accumulators of the C entries
 constexpr int STATIC_RESERVE = 1024;     // the kernel's static shared memory
 constexpr uint32_t SLEEP_DRAIN = 256;    // ns between polls of the drain warps (a period is ~8 rounds)
@@ -98,6 +101,7 @@ struct Args {
   int nmma;              // MMA N (multiple of 16, >= 16)
   int tmem_cols;         // two accumulator sets of nmma columns
   uint32_t lbo_a, lbo_b; // bytes between k-octets of the A / B digit buffers
+  int sort_bytes;        // SortBuf<2> or <4>
   uint32_t dig_a, dig_b; // bytes of one A / B digit buffer (A includes DPAD)
   double* partials;
   unsigned* counter;
@@ -228,7 +232,6 @@ template <int NP, typename TI>
 __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p) {
   constexpr int BN = NP < 8 ? NP : 8;  // B columns per drain block
   constexpr int NB = NP / BN;          // drain blocks
-  constexpr int NC = NP < NCMAX ? NP : NCMAX;
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);           // [MAXST] FP64 stage landed
   uint64_t* empty = full + MAXST;                                // [MAXST] FP64 stage consumed
@@ -246,9 +249,9 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
   int* Ecur = reinterpret_cast<int*>(smem + 256);                      // [32] A columns, then B
   int* pe = reinterpret_cast<int*>(smem + 384);                        // [2][32] a period's exponents
   int* ae = reinterpret_cast<int*>(smem + 640);                        // [32] exponents of the drain's sums
-  int* D = reinterpret_cast<int*>(smem + HDR);                         // [8 * NC][DSTRIDE]
-  double* cacc = reinterpret_cast<double*>(smem + HDR + SBYTES);
-  unsigned char* ring = smem + HDR + SBYTES + CBYTES;
+  int* D = reinterpret_cast<int*>(smem + HDR);                         // SortBuf: [8 * NC][STRIDE]
+  double* cacc = reinterpret_cast<double*>(smem + HDR + p.sort_bytes);
+  unsigned char* ring = smem + HDR + p.sort_bytes + CBYTES;
   unsigned char* dig = ring + (size_t)p.stages * p.stage_bytes;  // 1024-aligned by the host
   auto digA = [&](int d) { return dig + (size_t)d * (p.dig_a + p.dig_b); };
   auto digB = [&](int d) { return p.gram ? digA(d) : digA(d) + p.dig_a; };
@@ -418,38 +421,45 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
       }
       if (cnt && (done || chg || cnt == MAXSUM)) {  // levels -> FP64 accumulators
         // a few columns n at a time through shared memory; a thread then forms the eight level sums of a cell
+        auto sort = [&](auto buf) {
+          constexpr int NC = NP < decltype(buf)::NC ? NP : decltype(buf)::NC, STRIDE = decltype(buf)::STRIDE;
 #pragma unroll
-        for (int n0 = 0; n0 < NP; n0 += NC) {
-          if (qvalid) {
+          for (int n0 = 0; n0 < NP; n0 += NC) {
+            if (qvalid) {
 #pragma unroll
-            for (int j = 0; j < DIGITS; j++)
+              for (int j = 0; j < DIGITS; j++)
 #pragma unroll
-              for (int x = 0; x < NC; x++) D[(j * NC + x) * DSTRIDE + r] = acc[j * NP + n0 + x];
-          }
-          drainers_sync();
-          for (int e = dtid; e < M * min(NC, N - n0); e += NDRAIN * 32) {
-            const int mm = e % M, x = e / M;
-            const int* Dc = D + x * DSTRIDE + mm;
-            long long sv[8];
-#pragma unroll
-            for (int t = 0; t < DIGITS; t++) {
-              int sum = 0;  // |sum| <= 8 * MAXSUM * 2^24
-#pragma unroll
-              for (int i = 0; i <= t; i++) sum += Dc[(t - i) * NC * DSTRIDE + i * MP];
-              sv[t] = sum;
+                for (int x = 0; x < NC; x++) D[(j * NC + x) * STRIDE + r] = acc[j * NP + n0 + x];
             }
-            const long long vhi = (sv[0] << 24) + (sv[1] << 16) + (sv[2] << 8) + sv[3];
-            const long long vlo = (sv[4] << 24) + (sv[5] << 16) + (sv[6] << 8) + sv[7];
-            const int ea = ae[mm], eb = ae[(p.gram ? 0 : 16) + n0 + x];
-            const double v = fma((double)vlo, 0x1p-32, (double)vhi);  // in units of 2^(EA+EB-2080)
-            double& ca = cacc[(n0 + x) * M + mm];
-            // (one factor where it is in range, so that a small one of the two does not round v)
-            const int es = ea + eb - 2080;
-            ca = (unsigned)(es + 1022) <= 2045u ? fma(v, pow2i(es), ca)
-                                                : fma(v * pow2i(ea - 1040), pow2i(eb - 1040), ca);
+            drainers_sync();
+            for (int e = dtid; e < M * min(NC, N - n0); e += NDRAIN * 32) {
+              const int mm = e % M, x = e / M;
+              const int* Dc = D + x * STRIDE + mm;
+              long long sv[8];
+#pragma unroll
+              for (int t = 0; t < DIGITS; t++) {
+                int sum = 0;  // |sum| <= 8 * MAXSUM * 2^24
+#pragma unroll
+                for (int i = 0; i <= t; i++) sum += Dc[(t - i) * NC * STRIDE + i * MP];
+                sv[t] = sum;
+              }
+              const long long vhi = (sv[0] << 24) + (sv[1] << 16) + (sv[2] << 8) + sv[3];
+              const long long vlo = (sv[4] << 24) + (sv[5] << 16) + (sv[6] << 8) + sv[7];
+              const int ea = ae[mm], eb = ae[(p.gram ? 0 : 16) + n0 + x];
+              const double v = fma((double)vlo, 0x1p-32, (double)vhi);  // in units of 2^(EA+EB-2080)
+              double& ca = cacc[(n0 + x) * M + mm];
+              // (one factor where it is in range, so that a small one of the two does not round v)
+              const int es = ea + eb - 2080;
+              ca = (unsigned)(es + 1022) <= 2045u ? fma(v, pow2i(es), ca)
+                                                  : fma(v * pow2i(ea - 1040), pow2i(eb - 1040), ca);
+            }
+            drainers_sync();
           }
-          drainers_sync();
-        }
+        };
+        if (p.sort_bytes == SortBuf<4>::BYTES)
+          sort(SortBuf<4>{});
+        else
+          sort(SortBuf<2>{});
 #pragma unroll
         for (int x = 0; x < DIGITS * NP; x++) acc[x] = 0;
         cnt = 0;
@@ -740,7 +750,7 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   // a round starts at a multiple of 128 rows, so its bytes start 16-byte aligned with the operand
   const bool aligned = ((uintptr_t)A % 16 == 0) && (a.gram || (uintptr_t)B % 16 == 0);
   const bool dense = lda <= 2 * M + 16 && (a.gram || ldb <= 2 * N + 16);
-  const int64_t fixed = HDR + SBYTES + CBYTES + STATIC_RESERVE;
+  const int64_t fixed = HDR + SortBuf<2>::BYTES + CBYTES + STATIC_RESERVE;
   int64_t dstage = 0;
   a.stages = 0;
   for (int R = PERIOD / 128; R >= 1 && a.stages == 0; R /= 2) {
@@ -769,8 +779,13 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
     return SKINNY_UNSUPPORTED;
   }
   a.nrounds = (K + a.rr - 1) / a.rr;
-  const int smem2 =
-      (int)(fixed - STATIC_RESERVE + (int64_t)a.stages * a.stage_bytes + (int64_t)a.dstages * dstage);
+  int64_t smem2 = fixed + (int64_t)a.stages * a.stage_bytes + (int64_t)a.dstages * dstage;
+  a.sort_bytes = SortBuf<2>::BYTES;
+  if (smem2 + SortBuf<4>::BYTES - SortBuf<2>::BYTES <= h->dev.smem_optin) {
+    a.sort_bytes = SortBuf<4>::BYTES;
+    smem2 += SortBuf<4>::BYTES - SortBuf<2>::BYTES;
+  }
+  smem2 -= STATIC_RESERVE;
   const int64_t grid = std::max<int64_t>(1, std::min<int64_t>({a.nrounds, h->dev.sms, (int64_t)GROUP * MAXGROUPS}));
   Workspace& ws = h->ws[st];
   // CTA partials, then the group sums
@@ -781,19 +796,19 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   a.err = h->err;
   if (!in_f32) {
     switch (NP) {
-      case 1: return launch<1, double>(a, (int)grid, smem2, st);
-      case 2: return launch<2, double>(a, (int)grid, smem2, st);
-      case 4: return launch<4, double>(a, (int)grid, smem2, st);
-      case 8: return launch<8, double>(a, (int)grid, smem2, st);
-      case 16: return launch<16, double>(a, (int)grid, smem2, st);
+      case 1: return launch<1, double>(a, (int)grid, (int)smem2, st);
+      case 2: return launch<2, double>(a, (int)grid, (int)smem2, st);
+      case 4: return launch<4, double>(a, (int)grid, (int)smem2, st);
+      case 8: return launch<8, double>(a, (int)grid, (int)smem2, st);
+      case 16: return launch<16, double>(a, (int)grid, (int)smem2, st);
     }
   } else {
     switch (NP) {
-      case 1: return launch<1, float>(a, (int)grid, smem2, st);
-      case 2: return launch<2, float>(a, (int)grid, smem2, st);
-      case 4: return launch<4, float>(a, (int)grid, smem2, st);
-      case 8: return launch<8, float>(a, (int)grid, smem2, st);
-      case 16: return launch<16, float>(a, (int)grid, smem2, st);
+      case 1: return launch<1, float>(a, (int)grid, (int)smem2, st);
+      case 2: return launch<2, float>(a, (int)grid, (int)smem2, st);
+      case 4: return launch<4, float>(a, (int)grid, (int)smem2, st);
+      case 8: return launch<8, float>(a, (int)grid, (int)smem2, st);
+      case 16: return launch<16, float>(a, (int)grid, (int)smem2, st);
     }
   }
   set_error("split precision: unsupported N");
