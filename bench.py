@@ -329,12 +329,14 @@ def kernel_of(it, method):
         Mr, Nr = (2 * M, 2 * N) if it["dt"] == "c64" else (M, N)
         wide = Mr > 16 or Nr > 16
         nblk = ((Mr + 63) // 64) * ((Nr + 63) // 64)
-        auto_split = K >= 4096 and (Mr * Nr >= 256 or (Mr >= 8 and Nr >= 8)) and \
-            (not wide or Mr * Nr >= (128 if Mr <= 32 and Nr <= 32 else 320) * nblk)
+        auto_split = K >= 4096 and Mr >= 4 and Nr >= 4 and Mr * Nr >= 32 and \
+            K * Mr * Nr >= (1 << 22 if Mr >= 8 and Nr >= 8 else 3 << 22) and \
+            (not wide or Mr * Nr >= (128 if Mr <= 32 and Nr <= 32 else 256) * nblk) and \
+            not (it["dt"] == "c64" and wide and K * Mr * Nr <= 1 << 23)
         if fp64 and (method == "split" or (method == "auto" and auto_split)):
             return "split_wide_kernel" if wide else "split_tsmttsm_kernel"
         p2 = lambda x: 1 << (x - 1).bit_length()
-        cap = 16 if it["dt"] == "c64" else 64  # register tiles of the row-streaming kernel
+        cap = 16 if fp64 or K >= 1 << 20 else 64  # register tiles of the row-streaming kernel
         if M <= 8 and N <= 8 and p2(M) * p2(N) <= cap:
             return "tsmttsm_rows_kernel"
         return "tsmttsm_kernel"
@@ -342,6 +344,8 @@ def kernel_of(it, method):
     auto_split = K >= 8192 and (Mr * Nr >= 128 or (it["dt"] == "c64" and Mr * Nr >= 64)) and Nr >= 8 and Mr >= 4
     if fp64 and (method == "split" or (method == "auto" and auto_split)):
         return "split_tsmm_kernel"
+    if not fp64 and max(M, N) * it["s"] > 16:
+        return "tsmm_tile_kernel"
     return "tsmm_kernel"
 
 
