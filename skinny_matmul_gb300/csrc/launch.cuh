@@ -245,9 +245,13 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
   pl.ldb_s = gram ? pl.lda_s : (bulk ? ldb : N);
   if (!bulk) pl.vec = std::is_same<T, float>::value && pl.lda_s % 4 == 0 && pl.ldb_s % 4 == 0;
   pl.ntiles = (K + rows - 1) / rows;
-  const int nslots = G < 32 && (G & (G - 1)) == 0 ? TSMTTSM_THREADS / 32 : RS;
   const int64_t E = G * tm * tn;
-  const int64_t red = std::max<int64_t>(nslots > 1 ? nslots * E : 0, TSMTTSM_THREADS) * (int64_t)sizeof(Acc);
+  // shared memory of the reduction: full groups of cells have one row slice, a last group with fewer
+  // cells as many as fit the threads, whose sums need the more room (double-double Gram 89: 104 cells
+  // behind a group of 256, 123 008 bytes where the ring takes 91 520)
+  const int64_t Glast = Gall - (groups - 1) * TSMTTSM_THREADS;
+  const int64_t red = std::max(tsmttsm_red_entries((int)G, tm * tn), tsmttsm_red_entries((int)Glast, tm * tn)) *
+                      (int64_t)sizeof(Acc);
   pl.smem = (int)(SMEM_HEADER + std::max(stages * stage + SMEM_SLACK, red));
   int64_t grid = ctas;
   if (grid > pl.ntiles) grid = pl.ntiles;

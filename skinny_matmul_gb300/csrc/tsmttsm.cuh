@@ -109,6 +109,18 @@ __device__ __forceinline__ void cell_slice(const T* p, int band, T (&v)[W]) {
   }
 }
 
+// How many sums of each entry of G cells (TE entries each) a CTA joins in shared memory: one per warp
+// where the lanes of a warp hold a power of two of cells, else one per row slice
+__host__ __device__ __forceinline__ int tsmttsm_slots(int G) {
+  return G < 32 && (G & (G - 1)) == 0 ? TSMTTSM_THREADS / 32 : TSMTTSM_THREADS / G;
+}
+// Accumulators of shared memory behind the ring barriers that reducing those cells takes: the slots,
+// where there are several, and one per thread for the cross-CTA sum
+__host__ __device__ __forceinline__ int64_t tsmttsm_red_entries(int G, int TE) {
+  const int64_t slots = tsmttsm_slots(G), e = slots > 1 ? slots * G * TE : 0;
+  return e > TSMTTSM_THREADS ? e : TSMTTSM_THREADS;
+}
+
 // Cell c of the lower triangle of a square cell grid, row by row: (i, j), j <= i
 __host__ __device__ __forceinline__ void tri_cell(int c, int& i, int& j) {
   i = (int)((sqrtf(8.0f * (float)c + 1.0f) - 1.0f) * 0.5f);
@@ -269,10 +281,10 @@ __global__ void __launch_bounds__(TSMTTSM_THREADS, tsmttsm_ctas<Acc>(TM * TN)) t
   Acc* part = reinterpret_cast<Acc*>(p.partials) + (size_t)blockIdx.y * gridDim.x * NT * TE;
   Acc* mine = part + (size_t)blockIdx.x * E;
   Acc* red = reinterpret_cast<Acc*>(smem + SMEM_HEADER);
-  int base = 0, n = TE, nslots = RS, slot = rs;
+  const int nslots = tsmttsm_slots(G);
+  int base = 0, n = TE, slot = rs;
   bool owner = active;
   if (G < 32 && (G & (G - 1)) == 0) {  // every warp is active
-    nslots = NW;
     slot = warp;
     warp_halve<O, Acc, TE>(acc, G, lane, base, n, owner);
   }
