@@ -455,19 +455,25 @@ __global__ void __launch_bounds__(EIG_THREADS) svqb_eig_kernel(const double* __r
 
   const double* A0 = sh + cur;
 
-  // ascending eigenvalues: rank of each diagonal entry (ties broken by index)
+  // ascending eigenvalues: rank of each diagonal entry (ties broken by index; NaN ranks as infinity, so
+  // that the ranks are a permutation whatever the block holds)
+  auto eigenvalue = [&](int i) { return fmin(A0[slot_of(i, n) * (LD + 1)], HUGE_VAL); };
+  bool nan = false;
   for (int i = tid / 8; i < (M + 3) / 4 * 4; i += EIG_THREADS / 8) {  // whole warps, 8 lanes per entry
-    const double li = i < M ? A0[slot_of(i, n) * (LD + 1)] : 0.0;
+    const double li = i < M ? eigenvalue(i) : 0.0;
+    nan |= i < M && isnan(A0[slot_of(i, n) * (LD + 1)]);
     int rank = 0;
     for (int j = tid % 8; j < M; j += 8) {
-      const double lj = A0[slot_of(j, n) * (LD + 1)];
+      const double lj = eigenvalue(j);
       rank += (lj < li) || (lj == li && j < i);
     }
 #pragma unroll
     for (int o = 4; o >= 1; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
     if (i < M && tid % 8 == 0) order[rank] = i;
   }
-  __syncthreads();
+  // NaN or infinity in the block (and so on the Gram's diagonal): T is NaN throughout, as rotations by
+  // NaN would make it; M == 1 has none
+  nan = __syncthreads_or(nan && M > 1);
   // T[col*M + m] = V[m][src] * d[m] / sqrt(max(1e-15, l_src)), sign: largest |V[.][src]| positive
   // (8 lanes per column; equal magnitudes: the first)
   for (int col = tid / 8; col < (M + 3) / 4 * 4; col += EIG_THREADS / 8) {  // whole warps
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(EIG_THREADS) svqb_eig_kernel(const double* __r
         at = a2;
       }
     }
-    const double f = sg / sqrt(fmax(1.0e-15, A0[src * LD + src]));
+    const double f = nan ? HUGE_VAL - HUGE_VAL : sg / sqrt(fmax(1.0e-15, A0[src * LD + src]));
     if (col < M)
       for (int m = sub; m < M; m += 8) T[col * M + m] = V[m * LD + src] * d[m] * f;
   }

@@ -149,11 +149,12 @@ __global__ void __launch_bounds__(CTHREADS) svqbz_eig_kernel(const z2* __restric
     }
   }
 
+  // (NaN ranks as infinity, so that the ranks are a permutation whatever the block holds)
   for (int i = tid; i < M; i += CTHREADS) {
-    const double li = A[i * LD + i].x;
+    const double li = fmin(A[i * LD + i].x, HUGE_VAL);
     int rank = 0;
     for (int j = 0; j < M; j++) {
-      const double lj = A[j * LD + j].x;
+      const double lj = fmin(A[j * LD + j].x, HUGE_VAL);
       rank += (lj < li) || (lj == li && j < i);
     }
     order[rank] = i;
