@@ -36,6 +36,10 @@ static_assert(EIG_SIZE >= SVQB_MAX_M * EIG_LD, "a buffer holds the matrix");
 constexpr int EIG_MIXED_MIN = 8;
 // A pair of eigenvectors is refined to first order when its rotation is below this
 constexpr double EIG_SMALL = 1.0 / 1024.0;
+// and when the eigenvalues differ by more than this: far below the rounding level of a matrix of unit
+// diagonal, far above the smallest FP32 number with a finite reciprocal (2^-128), which null vectors of
+// dependent columns, whose eigenvalues are 1e-33 to 1e-50 apart, are not
+constexpr double EIG_GAP = 0x1p-100;
 
 // Round-robin order in slots: pair l of a round is slots l and 32 + l.  From one round to the next the
 // players move one pair on, p to the pair below, q to the pair above, with player n - 1 fixed in slot
@@ -410,7 +414,7 @@ __global__ void __launch_bounds__(SVQB_THREADS) eig_update_kernel(const double* 
         if (refine) {
           const double s = S[k * M + j], gap = lam[j] - lam[k];
           const double num = s - lam[j] * g, lim = EIG_SMALL * fabs(gap);
-          if (fabs(num) <= lim && fabs(s - lam[k] * g) <= lim && gap != 0.0) return num * (double)(1.0f / (float)gap);
+          if (fabs(num) <= lim && fabs(s - lam[k] * g) <= lim && fabs(gap) > EIG_GAP) return num * (double)(1.0f / (float)gap);
         }
         return -0.5 * g;
       },
