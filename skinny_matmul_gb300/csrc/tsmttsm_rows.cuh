@@ -43,22 +43,41 @@ struct RowsArgs {
   unsigned* counter;
 };
 
-// W values of one row (zero beyond n or for a row past the end)
+template <typename V>
+__host__ __device__ __forceinline__ V read_only(const V* p) {
+#ifdef __CUDA_ARCH__
+  return __ldg(p);
+#else
+  return *p;
+#endif
+}
+
+// W values of one row (zero beyond n or for a row past the end); nothing but those n is read, for the last
+// row may end the allocation
 template <typename T, int W>
-__device__ __forceinline__ void row_vals(const T* __restrict__ row, int n, bool ok, bool vec, T (&v)[W]) {
+__host__ __device__ __forceinline__ void row_vals(const T* __restrict__ row, int n, bool ok, bool vec, T (&v)[W]) {
   if constexpr (std::is_same<T, double>::value && W >= 2) {
     if (vec) {
 #pragma unroll
       for (int x = 0; x < W; x += 2) {
-        const double2 d = ok ? __ldg(reinterpret_cast<const double2*>(row + x)) : make_double2(0.0, 0.0);
-        v[x] = x < n ? d.x : 0.0;
-        v[x + 1] = x + 1 < n ? d.y : 0.0;
+        double2 d = make_double2(0.0, 0.0);
+        if (ok && x + 1 < n)
+          d = read_only(reinterpret_cast<const double2*>(row + x));
+        else if (ok && x < n)
+          d.x = read_only(row + x);
+        v[x] = d.x;
+        v[x + 1] = d.y;
       }
       return;
     }
   }
 #pragma unroll
-  for (int x = 0; x < W; x++) v[x] = (ok && x < n) ? row[x] : tzero<T>();
+  for (int x = 0; x < W; x++) {
+    if (ok && x < n)
+      v[x] = row[x];
+    else
+      v[x] = T{};
+  }
 }
 
 template <typename T, typename Acc, int TM, int TN, int U>
