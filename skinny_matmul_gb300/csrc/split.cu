@@ -45,7 +45,8 @@
 //   * Cross-CTA finish in two levels: CTA partials in FP64; the last CTA of each group of 16
 //     (ticket) sums its group in CTA order, the last group sums the group sums in group order
 //     and applies alpha/beta (deterministic).
-// Inputs must be finite (Inf/NaN have no fixed-point form).
+//   * Infinities and NaN have no fixed-point form: a column that holds one gets the exponent NONFINITE, whose
+//     power of two is NaN, and so are the entries of C that it enters.
 
 #include <cstring>
 
@@ -67,6 +68,8 @@ constexpr int WPROD = NSLICE + NDRAIN, WMMA = WPROD + 1;
 constexpr int THREADS = (WMMA + 3) * 32;
 constexpr int SLICERS = NSLICE * 32;
 constexpr int HEAD = 2;        // exponent headroom granted when a column's exponent is raised
+constexpr int EMAX = 2046;     // largest exponent field of a finite number, and of a column of such
+constexpr int NONFINITE = 6000;  // exponent of a column with an infinity or NaN: out of the range of any sum
 constexpr int MAXST = 4;       // FP64 stages (at most)
 constexpr int MAXDST = 3;      // digit stages (at most)
 constexpr int DPAD = 128 * 16; // slack after an A digit buffer: the MMA reads 128 rows per k-octet
@@ -163,7 +166,8 @@ __device__ __forceinline__ uint32_t exp_field(double x) {
   return nz ? (ef ? ef : 1u) : 0u;
 }
 
-__device__ __forceinline__ double pow2i(int e) {  // 2^e for e in [-1022, 1023], clamped outside
+__device__ __forceinline__ double pow2i(int e) {  // 2^e for e in [-1022, 1023], clamped outside; NONFINITE: NaN
+  if (e > NONFINITE / 2) return __hiloint2double(0x7FF80000, 0);
   e = e < -1022 ? -1022 : (e > 1023 ? 1023 : e);
   return __hiloint2double((e + 1023) << 20, 0);
 }
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(THREADS, 1) split_tsmttsm_kernel(const Args p)
           break;
         }
         // a new period: raise the exponents of the columns that met larger elements
-        if (exceed) atomicMax(&Ecur[(isB ? 16 : 0) + col], (int)eu + HEAD);
+        if (exceed) atomicMax(&Ecur[(isB ? 16 : 0) + col], (int)eu > EMAX ? NONFINITE : min((int)eu + HEAD, EMAX));
         pp++;
         bool ok2 = true;  // the period's exponent slot and accumulator set held period pp - 2
         if (pp >= 2) ok2 = wait_ab(&drained[pp & 1], (uint32_t)(((pp - 2) >> 1) & 1), abort_f, p.err);

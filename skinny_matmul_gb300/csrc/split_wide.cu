@@ -62,7 +62,8 @@
 //     diagonal quadrants of the 64 x 64 accumulators then hold the sums over the two row halves
 //     (the off-diagonal quadrants pair different rows and are not read), so a 32-wide product
 //     uses every slicer and every MMA column, and the halves are added at the end.
-// Inputs must be finite (Inf/NaN have no fixed-point form).
+//   * Infinities and NaN have no fixed-point form: a column that holds one gets the exponent NONFINITE, whose
+//     power of two is NaN, and so are the entries of C that it enters.
 #include <atomic>
 #include <cstring>
 
@@ -78,6 +79,8 @@ constexpr int PSTAGES = 8;   // stages per accumulation period (128 rows: exact 
 constexpr int DSLOTS = 3;    // digit slots
 constexpr int MAXR = 8;      // FP64 stages (at most)
 constexpr int HEAD = 4;      // exponent headroom granted when a column's exponent is raised
+constexpr uint32_t EMAX = 2046;  // largest exponent field of a finite number, and of a column of such
+constexpr int NONFINITE = 6000;  // exponent of a column with an infinity or NaN: out of the range of any sum
 constexpr int SW = 16;       // slicer warps: 0-15
 constexpr int DW = 8;        // drain warps: 16-23
 constexpr int WPROD = SW + DW, WMMA = WPROD + 1;  // producer warps: WPROD and, for rows copied one by one, two more
@@ -209,7 +212,8 @@ __device__ __forceinline__ uint32_t exp_field(double x) {
   return e == 0 && (mh | (uint32_t)__double2loint(x)) ? 1u : e;
 }
 
-__device__ __forceinline__ double pow2i(int e) {  // 2^e, clamped to the normal range
+__device__ __forceinline__ double pow2i(int e) {  // 2^e, clamped to the normal range; NONFINITE: NaN
+  if (e > NONFINITE / 2) return __hiloint2double(0x7FF80000, 0);
   e = e < -1022 ? -1022 : (e > 1023 ? 1023 : e);
   return __hiloint2double((e + 1023) << 20, 0);
 }
@@ -632,9 +636,9 @@ __global__ void __launch_bounds__(THREADS, 1) split_wide_kernel(const Args p) {
         }
         __syncwarp();
         if (cvalid && e > Ecur) {
-          if (sub == 0)
-            rec[(isB ? 64 : 0) + c] = ((uint64_t)(uint32_t)ls << 32) | (uint64_t)((Ecur << 16) | (e + HEAD));
-          Ecur = e + HEAD;
+          const uint32_t raise = e > EMAX ? (uint32_t)NONFINITE : min(e + HEAD, EMAX);
+          if (sub == 0) rec[(isB ? 64 : 0) + c] = ((uint64_t)(uint32_t)ls << 32) | (uint64_t)((Ecur << 16) | raise);
+          Ecur = raise;
         }
         raised = ls;
         vflag[ls & 3] = ls + 1;
