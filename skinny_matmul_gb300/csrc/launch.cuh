@@ -8,6 +8,7 @@
 #pragma once
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <string>
 
 #include "skinny.h"
@@ -135,6 +136,12 @@ skinny_status tsmttsm_dispatch(const TsmttsmPlan& pl, const TsmttsmArgs<T>& a, c
   return SKINNY_UNSUPPORTED;
 }
 
+// FP32 storage summed in FP64 (the double-double method of float and complex float)
+template <typename T, typename Acc>
+constexpr bool widens() {
+  return sizeof(Acc) == 2 * sizeof(T) && !std::is_same<Acc, dd>::value && !std::is_same<Acc, zdd>::value;
+}
+
 // Clocks one SM takes for `rows` rows with TM x TN cells, and for its reduction (model).  FP64-pipe
 // types: a warp instruction holds the pipe of its SM partition (one of 4) for ~68 clocks, so the
 // time is the busiest partition's warps times the tile, padding included, and reducing the CTA
@@ -148,7 +155,15 @@ double tsmttsm_tile_cost(int64_t M, int64_t N, int tm, int tn, int64_t cells, bo
   if (!fp32_sums<Acc>()) {
     const double macs = std::is_same<Acc, zdd>::value ? 32 : std::is_same<Acc, dd>::value ? 8 : sizeof(Acc) / 4;
     const double adds = std::is_same<Acc, zdd>::value ? 40 : std::is_same<Acc, dd>::value ? 20 : sizeof(Acc) / 8;
-    return 68.0 * busiest * t * (macs * (sizeof(Acc) == 8 ? 0.5 : 1.0) * rows / RS + 1.5 * adds);
+    const double ops = t * macs * (sizeof(Acc) == 8 ? 0.5 : 1.0);
+    if constexpr (widens<T, Acc>()) {
+      // FP32 values are widened on the FP64 pipe too: 1 x 1 cells spend two thirds of it on that.  Large cells
+      // have many row slices, whose passes over a CTA's rows are counted whole.
+      const int ctas = rows < 256.0 ? 1 : tsmttsm_ctas<Acc>(t);
+      const double passes = std::ceil(rows / ctas / RS), widen = (double)(sizeof(T) / 4) * (tm + tn);
+      return 68.0 * busiest * ctas * ((ops + widen) * passes + 1.5 * adds * t);
+    }
+    return 68.0 * busiest * (ops * rows / RS + 1.5 * adds * t);
   }
   const double flops = std::is_same<Acc, float>::value ? 1 : 4;
   const double fma = busiest * t * flops;
@@ -157,19 +172,24 @@ double tsmttsm_tile_cost(int64_t M, int64_t N, int tm, int tn, int64_t cells, bo
   return std::max(step / RS, row_bytes / 44.0) * rows + t * 8.0 * busiest;
 }
 
+// Whole rows of both operands, leading dimension and all, are bulk copied: they start on 16 bytes (a tile holds a
+// multiple of 16 rows) and carry little besides the columns that count
+inline bool bulk_rows(int64_t M, int64_t N, const void* A, int64_t lda, const void* B, int64_t ldb, bool gram) {
+  return (uintptr_t)A % 16 == 0 && lda <= 2 * M + 16 && (gram || ((uintptr_t)B % 16 == 0 && ldb <= 2 * N + 16));
+}
+
 template <typename T, typename Acc>
 skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t K, const void* A,
                            int64_t lda, const void* B, int64_t ldb, bool gram, const LaunchOpts& o,
                            TsmttsmPlan& pl) {
   const int cap = tile_cap<Acc>();
   const int64_t s = sizeof(T);
-  const bool aligned = ((uintptr_t)A % 16 == 0) && (gram || (uintptr_t)B % 16 == 0);
-  const bool dense = lda <= 2 * M + 16 && (gram || ldb <= 2 * N + 16);
+  const bool whole = bulk_rows(M, N, A, lda, B, ldb, gram);
   // shared row strides: ld when bulk-copied, dense (M / N) when loaded by threads
   const int64_t row_bytes_bulk = (lda + (gram ? 0 : ldb)) * s;
   const int64_t row_bytes_dense = (M + (gram ? 0 : N)) * s;
-  const int64_t rb = (aligned && dense) ? row_bytes_bulk : row_bytes_dense;
-  const int64_t las = aligned && dense ? lda : M, lbs = gram ? las : (aligned && dense ? ldb : N);
+  const int64_t rb = whole ? row_bytes_bulk : row_bytes_dense;
+  const int64_t las = whole ? lda : M, lbs = gram ? las : (whole ? ldb : N);
   pl.vec = std::is_same<T, float>::value && las % 4 == 0 && lbs % 4 == 0;
 
   // the tile: the cheapest one whose cells fit one group of threads; beyond, the largest
@@ -180,7 +200,7 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
   for (int tm = 1; tm <= pm; tm *= 2)
     for (int tn = 1; tn <= pn; tn *= 2) {
       if (tm * tn > cap || (gram && tm != tn)) continue;
-      if (sizeof(Acc) == 8 && tm * tn > 16) continue;
+      if (sizeof(Acc) == 8 && tm * tn > 16 && !widens<T, Acc>()) continue;
       const int64_t gm = (M + tm - 1) / tm, gn = (N + tn - 1) / tn;
       const int64_t cells = gram ? gm * (gm + 1) / 2 : gm * gn;
       if (cells > TSMTTSM_THREADS) continue;
@@ -217,19 +237,35 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
   if (rows <= 0) {
     // FP64-pipe types: 16 KB.  FP32: a third of the CTA's shared memory, for a tile of 16 KB is
     // only a few rows per thread and the hand-offs show (13 x 7, 3.4e6 rows: 102 us; 69 with 32 KB)
-    const int64_t most = fp32_sums<Acc>() ? (int64_t)208 * 1024 / bps / 3 - 256 : 16384;
+    // and widened types 32 KB, for the choice of rows below
+    const int64_t most = fp32_sums<Acc>() ? (int64_t)208 * 1024 / bps / 3 - 256 : widens<T, Acc>() ? 32768 : 16384;
     rows = (int)std::max<int64_t>(16, std::min<int64_t>(1024, most / rb / 16 * 16));
     // the same whole number of tiles for every CTA (rows are handed out in 16s), at least two
     // each where K allows, so that copies and sums overlap
     const int64_t per_cta = std::max<int64_t>((K + ctas - 1) / ctas, 1);
     const int64_t n = std::max<int64_t>((per_cta + rows - 1) / rows, per_cta >= 64 ? 2 : 1);
+    const int most_rows = (int)std::min<int64_t>(rows, round_up((per_cta + 1) / (per_cta >= 64 ? 2 : 1), 16));
     rows = (int)std::min<int64_t>(rows, round_up((per_cta + n - 1) / n, 16));
+    // widened types take the largest tiles, so the most row slices: down to three quarters of the rows that
+    // fit, the ones with the fewest passes of the slices over a CTA's tiles, a hand-off counting a quarter
+    // (144 rows for 128 slices are two passes, the second nearly empty: complex FP32 7 x 7, 2^20 rows:
+    // 749 us, 585 with 128 rows; FP64 and FP32 lose as much as they gain by it, up to 10 %)
+    if (widens<T, Acc>()) {
+      int64_t fewest = -1;
+      for (int r = most_rows; r >= 16 && 4 * r >= 3 * most_rows; r -= 16) {
+        const int64_t tiles = ((K + r - 1) / r + ctas - 1) / ctas, passes = tiles * (4 * ((r + RS - 1) / RS) + 1);
+        if (fewest < 0 || passes < fewest) {
+          fewest = passes;
+          rows = r;
+        }
+      }
+    }
   }
   rows = (int)round_up(rows < RS ? RS : rows, 16);
   const int64_t stage_a = round_up(rows * las * s, 128);
   const int64_t stage_b = gram ? 0 : round_up(rows * lbs * s, 128);
   const int64_t stage = stage_a + stage_b;
-  const bool bulk = aligned && dense && stage <= 65536 && K > rows;
+  const bool bulk = whole && stage <= 65536 && K > rows;
   const int64_t budget = (int64_t)dev.smem_optin - SMEM_HEADER - 1024;
   int stages = (int)std::min<int64_t>(TSMTTSM_MAX_STAGES, (208 * 1024 / bps) / std::max<int64_t>(stage, 1));
   if (stages < 2) stages = 2;
@@ -263,31 +299,40 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
 }
 
 // ----------------------------------------------------------------- TSMTTSM, narrow products
-// Register-tile entries a thread of the row-streaming kernel may hold: 64 for sums on the FP32 pipe
-// (8 x 8), 16 for FP64 (8 x 8 on the ring kernel: 11.1 us against 14.6 at 2^14 rows, the same at
+// Register-tile entries a thread of the row-streaming kernel may hold: 64 for FP32 and complex FP32 storage
+// (8 x 8; complex FP32 summed in FP64: 16), 16 for FP64 (8 x 8 on the ring kernel: 11.1 us against 14.6 at 2^14 rows, the same at
 // 2^20; 7 x 7 116 us against 143 at 1.2e6 rows), 16 for other 16-byte accumulators (complex FP64, double-double), 4 for
 // 32-byte ones (complex double-double).
-template <typename Acc>
+template <typename T, typename Acc>
 constexpr int rows_cap() {
-  return fp32_sums<Acc>() ? 64 : (sizeof(Acc) <= 16 ? 16 : 4);
+  return fp32_sums<Acc>() || (widens<T, Acc>() && sizeof(Acc) == 8) ? 64 : (sizeof(Acc) <= 16 ? 16 : 4);
 }
 
 // The row-streaming kernel takes a product when both padded widths are <= 8 and their tile fits
-// rows_cap; an autotuned row-tile size asks for the ring kernel instead.  FP32-pipe tiles above 16
-// entries stay with it below 2^20 rows (8 x 8 FP32: 5.1 us against 7.6 at 2^14 rows, 10.8 against
-// 12.3 at 2^18, the same at 2^20; 70 against 55 at 2^22: 64 sums a thread leave few loads in flight).
+// rows_cap; an autotuned row-tile size asks for the ring kernel instead.  Tiles above 16 entries
+//   * in double-double, from 2^16 rows on, go to it where the ring could not be filled by bulk copies (columns out
+//     of a wide block, 2^20 rows, L2 flushed, ring / rows: 6 x 6 226/187 us, 8 x 8 282/183);
+//   * FP32-pipe tiles stay with it below 2^20 rows (8 x 8 FP32: 5.1 us against 7.6 at 2^14 rows, 10.8
+//     against 12.3 at 2^18, the same at 2^20; 70 against 55 at 2^22: 64 sums a thread leave few loads in flight);
+//   * and FP32 summed in FP64 goes to the ring (6 x 6, 2^14 rows: 11.9 us against 15.1; 2^20: 171 against 178), but
+//     for long Gram products of 7 or 8 columns, one 8 x 8 cell there too (8 x 8, 2^18 rows: 80 against 69).
 template <typename T, typename Acc>
-bool rows_eligible(int64_t M, int64_t N, int64_t K, bool gram, const LaunchOpts& o) {
+bool rows_eligible(int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb, bool gram,
+                   const LaunchOpts& o) {
   if (o.rows_per_tile > 0 || M < 1 || N < 1 || M > 8 || N > 8) return false;
   int tm = pow2ceil(M), tn = pow2ceil(N);
   if (gram) tm = tn = std::max(tm, tn);
-  return tm * tn <= rows_cap<Acc>() && (tm * tn <= 16 || K < (1 << 20));
+  if (tm * tn > rows_cap<T, Acc>()) return false;
+  if (tm * tn <= 16) return true;
+  const bool whole = bulk_rows(M, N, A, lda, B, ldb, gram);
+  if (widens<T, Acc>()) return whole ? gram && M >= 7 && K >= (1 << 17) : K >= (1 << 16);
+  return K < (1 << 20);
 }
 
 template <typename T, typename Acc, int TM, int TN>
 skinny_status tsmttsm_rows_launch(RowsArgs<T>& a, const DeviceInfo& dev, Workspace& ws, int bps_opt,
                                   cudaStream_t st) {
-  if constexpr (TM * TN > rows_cap<Acc>()) {
+  if constexpr (TM * TN > rows_cap<T, Acc>()) {
     set_error("tsmttsm: register tile too large for the accumulator type");
     return SKINNY_UNSUPPORTED;
   } else {
@@ -365,7 +410,7 @@ skinny_status tsmttsm_run(const DeviceInfo& dev, Workspace& ws, int* err, cudaSt
                           const T* B, int64_t ldb, T beta, bool beta_zero, T* C, int64_t ldc,
                           const LaunchOpts& o) {
   const bool gram = (A == B) && (lda == ldb) && (M == N);
-  if (rows_eligible<T, Acc>(M, N, K, gram, o))
+  if (rows_eligible<T, Acc>(M, N, K, A, lda, B, ldb, gram, o))
     return tsmttsm_rows_run<T, Acc>(dev, ws, st, M, N, K, A, lda, alpha, B, ldb, beta, beta_zero, C, ldc, gram, o);
   TsmttsmPlan pl;
   skinny_status s = tsmttsm_plan<T, Acc>(dev, M, N, K, A, lda, B, ldb, gram, o, pl);
