@@ -336,7 +336,7 @@ def kernel_of(it, method):
         if fp64 and (method == "split" or (method == "auto" and auto_split)):
             return "split_wide_kernel" if wide else "split_tsmttsm_kernel"
         p2 = lambda x: 1 << (x - 1).bit_length()
-        cap = 16 if fp64 or K >= 1 << 20 else 64  # register tiles of the row-streaming kernel
+        cap = 64 if not fp64 and K < 1 << 20 else 32 if not fp64 and K < 3 << 19 else 16  # register tiles of the row-streaming kernel
         if M <= 8 and N <= 8 and p2(M) * p2(N) <= cap:
             return "tsmttsm_rows_kernel"
         return "tsmttsm_kernel"

@@ -310,10 +310,11 @@ constexpr int rows_cap() {
 
 // The row-streaming kernel takes a product when both padded widths are <= 8 and their tile fits
 // rows_cap; an autotuned row-tile size asks for the ring kernel instead.  Tiles above 16 entries
-//   * in double-double, from 2^16 rows on, go to it where the ring could not be filled by bulk copies (columns out
-//     of a wide block, 2^20 rows, L2 flushed, ring / rows: 6 x 6 226/187 us, 8 x 8 282/183);
-//   * FP32-pipe tiles stay with it below 2^20 rows (8 x 8 FP32: 5.1 us against 7.6 at 2^14 rows, 10.8
-//     against 12.3 at 2^18, the same at 2^20; 70 against 55 at 2^22: 64 sums a thread leave few loads in flight);
+//   * go to it where the ring could not be filled by bulk copies (columns out of a wide block, 2^20 rows, L2 flushed,
+//     ring / rows: FP32 6 x 6 76/52 us, in double-double, from 2^16 rows on, 226/187, 8 x 8 282/183);
+//   * else FP32-pipe tiles stay with it below 2^20 rows (8 x 8 FP32: 5.1 us against 7.6 at 2^14 rows, 10.8
+//     against 12.3 at 2^18, the same at 2^20; 70 against 55 at 2^22: 64 sums a thread leave few loads in flight),
+//     32 entries below 3 * 2^19 (5 x 3 FP32, 2^20 rows: 16.8 against 19.7; the same at 2^21);
 //   * and FP32 summed in FP64 goes to the ring (6 x 6, 2^14 rows: 11.9 us against 15.1; 2^20: 171 against 178), but
 //     for long Gram products of 7 or 8 columns, one 8 x 8 cell there too (8 x 8, 2^18 rows: 80 against 69).
 template <typename T, typename Acc>
@@ -326,7 +327,7 @@ bool rows_eligible(int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, 
   if (tm * tn <= 16) return true;
   const bool whole = bulk_rows(M, N, A, lda, B, ldb, gram);
   if (widens<T, Acc>()) return whole ? gram && M >= 7 && K >= (1 << 17) : K >= (1 << 16);
-  return K < (1 << 20);
+  return !whole || K < (tm * tn <= 32 ? 3 << 19 : 1 << 20);
 }
 
 template <typename T, typename Acc, int TM, int TN>
