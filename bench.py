@@ -344,7 +344,7 @@ def kernel_of(it, method):
     auto_split = K >= 8192 and (Mr * Nr >= 128 or (it["dt"] == "c64" and Mr * Nr >= 64)) and Nr >= 8 and Mr >= 4
     if fp64 and (method == "split" or (method == "auto" and auto_split)):
         return "split_tsmm_kernel"
-    if not fp64 and max(M, N) * it["s"] > 16:
+    if not fp64 and max(M, N) * it["s"] > 16 and not (M == 8 and N <= 2):  # dense FP32, widths powers of two
         return "tsmm_tile_kernel"
     return "tsmm_kernel"
 

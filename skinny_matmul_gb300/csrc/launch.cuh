@@ -492,15 +492,32 @@ skinny_status tsmm_tile_launch(const TsmmTileArgs<T>& a, int bps, int sms, int s
   return SKINNY_OK;
 }
 
-// The tiled kernel for float and complex float; false: the shape is left to tsmm_kernel (at most 4
-// columns in and out, which that streams at 0.75 of HBM rate, more than 128 outputs, or a tile that
-// does not fit).  Rows per thread: 8 where the FMA pipe is near (more than 16 columns of output), 4
-// otherwise, fewer while a CTA's ring is above 110 KB (two CTAs per SM) or SMs would go without rows.
+// Whether tsmm_kernel, whose threads walk a row each, is the better one for float and complex float (us, walking /
+// tiled, 2^20 rows, L2 flushed):
+//   * at most 16 bytes in and out, which it streams at 0.75 of HBM rate;
+//   * few columns out of rows that share cache lines (at most 128 bytes apart) and cannot be copied 16 bytes at a
+//     time: FP32 9 x 2 12.5/18.6, 16 x 1 in rows of 17 21/28.5, 24 x 3 the same; complex 9 x 1 in rows of 10 1.1x;
+//   * complex FP32 up to 6 x 2 also out of wide blocks (4 x 2, beta, 2^18 rows: 1.5x);
+//   * complex FP32, 5 to 9 outputs that do not fill the cells, from 2^17 packed rows that are not aligned: from 16 columns
+//     in on (33 x 9, 2^18 rows, L2 warm: 39/47; 17 x 5 1.2x; but 17 x 8 0.95x, 20 x 12 0.7x, 33 x 9 at 2^14 rows 0.8x),
+//     with beta and an odd number of outputs from 7 on (9 x 5 39.5/45; without 35/38).
+template <typename T>
+bool tsmm_walks(int M, int N, int np, int64_t K, int64_t lda, bool vec_a, bool beta) {
+  if (M * (int)sizeof(T) <= 16 && N * (int)sizeof(T) <= 16) return true;
+  const bool lines = lda * (int64_t)sizeof(T) <= 128;
+  if (sizeof(T) == 4) return lines && (vec_a ? N <= (beta ? 2 : 1) && M <= 8 : N <= 3 || (N == 4 && M > 8));
+  if ((N <= 2 && M <= 6) || (lines && N <= 3 && M <= (vec_a ? 4 : 9))) return true;
+  return K >= (1 << 17) && !vec_a && lda <= M + 8 && N >= 5 && N <= 9 && np > N && M >= (beta && N % 2 ? 7 : 16);
+}
+
+// The tiled kernel for float and complex float; false: the shape is left to tsmm_kernel (the rule above, more than
+// 128 outputs, or a tile that does not fit).  Rows per thread: 8 where the FMA pipe is near (more than 16
+// columns of output), 4 otherwise, fewer while a CTA's ring is above 110 KB (two CTAs per SM) or SMs would go
+// without rows.
 template <typename T>
 bool tsmm_tile_run(const DeviceInfo& dev, cudaStream_t st, const TsmmArgs<T>& t, const LaunchOpts& o, skinny_status& s) {
   constexpr int V = 16 / (int)sizeof(T);
   const int M = t.M, N = t.N;
-  if (M * (int)sizeof(T) <= 16 && N * (int)sizeof(T) <= 16) return false;
   TsmmTileArgs<T> a;
   a.t = t;
   a.t.gn = pow2ceil((N + V - 1) / V);
@@ -510,6 +527,7 @@ bool tsmm_tile_run(const DeviceInfo& dev, cudaStream_t st, const TsmmArgs<T>& t,
   a.stride = (chunks % 2 ? chunks : chunks + 1) * V;
   a.vec_a = M % V == 0 && t.lda % V == 0 && (uintptr_t)t.A % 16 == 0;
   a.vec_c = t.ldc % V == 0 && (uintptr_t)t.C % 16 == 0;
+  if (tsmm_walks<T>(M, N, a.t.np, t.K, t.lda, a.vec_a != 0, !t.beta_zero && !t.fold)) return false;
   const int64_t bs = (int64_t)M * a.t.np * sizeof(T);
   const int RP = TSMM_THREADS / a.t.gn;
   auto smem = [&](int R) { return bs + (int64_t)TSMM_TILE_STAGES * RP * R * a.stride * sizeof(T); };
