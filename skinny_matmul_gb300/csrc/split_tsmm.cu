@@ -62,18 +62,18 @@ constexpr int NSL = 8;
 __host__ __device__ constexpr int epi_groups(int nw) { return (nw - NSL) / 4; }
 constexpr int MAXAST = 3;                 // A' stages (at most)
 constexpr int CHUNK = 4;                  // output columns an epilogue warp converts at a time
-constexpr int CHUNK_BYTES = ROWS * CHUNK * 8;  // old C of one chunk
+constexpr int CRING = ROWS * CHUNK * 8;   // bytes of old C per group and unit of c_depth (one FP64 chunk, two of FP32)
 constexpr uint32_t SLEEP_MMA = 32;        // ns between polls of the MMA thread
 // Per contraction width MP: the ring of row-exponent records (tiles), the header (barriers, TMEM
 // slot, column exponents, row exponents; a multiple of 1024), and the old-C chunks each epilogue
 // warp group keeps in flight.  At MP = 64 B' (64 KB at N = 64) and one A' stage (128 KB) leave
-// 35 KB: a 3 KB header and two chunks per group fill the 227 KB exactly.
+// 35 KB: a 3 KB header and four chunks per group fill the 227 KB exactly.
 template <int MP>
 __host__ __device__ constexpr int row_ring() { return MP == 64 ? 4 : 8; }
 template <int MP>
 __host__ __device__ constexpr int hdr_bytes() { return MP == 64 ? 3072 : 5120; }
 template <int MP>
-__host__ __device__ constexpr int c_depth() { return MP == 32 ? 6 : 4; }
+__host__ __device__ constexpr int c_depth() { return MP == 32 ? 5 : 4; }
 
 struct Args {
   const void* A;    // storage type T of the kernel (double or float), as B and C
@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
   constexpr int NEP = NW - NSL, EG = epi_groups(NW);
   constexpr int TPS = NSL * 32 / ROWS;  // slicer threads per row (2 or 4)
   constexpr int PART = MP / TPS;        // A values per slicer thread
-  constexpr int CD = c_depth<MP>();    // old-C chunks in flight per epilogue thread
+  // old-C chunks in flight per epilogue thread, and the bytes of one (FP32 48 x 48, odd leading dimension, 2^18 rows:
+  // 242 us with as many chunks as FP64 in slots of twice their size, 200)
+  constexpr int CD = c_depth<MP>() * 8 / (int)sizeof(T), CHUNK_BYTES = ROWS * CHUNK * (int)sizeof(T);
   constexpr int RE = row_ring<MP>(), HDR = hdr_bytes<MP>();
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* afull = reinterpret_cast<uint64_t*>(smem);          // [MAXAST] A' stage written
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
   int* erow = reinterpret_cast<int*>(smem + 1024);              // [RE][ROWS] row exponents
   unsigned char* bdig = smem + HDR;                             // B' (1024-aligned)
   unsigned char* adig = bdig + p.bbytes;                        // A' stages
-  unsigned char* cbuf = adig + (size_t)p.nast * p.astage;       // [EG groups][CD][ROWS][8 doubles] old C
+  unsigned char* cbuf = adig + (size_t)p.nast * p.astage;       // [EG groups][CD][ROWS][CHUNK] old C
   const int M = p.M, N = p.N, NB = p.NB;
   // B' per block of NB output columns: rows j * NB + n (digit j + 1 of column n), K-major over
   // m in octets of 8 rows x 16 bytes (no swizzle); bytes between k-octets and between blocks:
@@ -577,7 +579,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
         const bool live = pf_row < p.K;
         const T* src = pf_src + CHUNK * pf_c;
         const int left = N - CHUNK * pf_c;
-        unsigned char* dst = cbuf + (uint32_t)(eg * CD + pf_s) * CHUNK_BYTES + r * (CHUNK * 8);
+        unsigned char* dst = cbuf + (uint32_t)(eg * CD + pf_s) * CHUNK_BYTES + r * (CHUNK * (int)sizeof(T));
         constexpr int PER16 = 16 / (int)sizeof(T);  // elements per 16-byte piece
         if (p.vecc) {
 #pragma unroll
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
           for (int x = 0; x < CHUNK; x++) {
             const uint32_t bytes = (live && left > x) ? (uint32_t)sizeof(T) : 0u;
             if constexpr (sizeof(T) == 8)
-              cp_async8(dst + 8 * x, bytes ? (const void*)(src + x) : p.C, bytes);
+              cp_async8(dst + (int)sizeof(T) * x, bytes ? (const void*)(src + x) : p.C, bytes);
             else
               cp_async4(dst + 4 * x, bytes ? (const void*)(src + x) : p.C, bytes);
           }
@@ -640,7 +642,7 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
         const uint32_t tb = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(k * 8 * NB);
         const int c_hi = min(CH, (cb + 1) * cpb);
         for (; c < c_hi; c += EG) {
-          const unsigned char* cs = cbuf + (uint32_t)(eg * CD + gs) * CHUNK_BYTES + r * (CHUNK * 8);
+          const unsigned char* cs = cbuf + (uint32_t)(eg * CD + gs) * CHUNK_BYTES + r * (CHUNK * (int)sizeof(T));
           if constexpr (HASC) {
             issue();  // into the slot of the last chunk, read in full already
             if (++gs == CD) gs = 0;
@@ -816,11 +818,13 @@ skinny_status split_tsmm_t(skinny_handle h, bool cplx, bool f32, int64_t M, int6
   // contraction width 16, more than 16 columns out: 24 warps
   const int nw = MP == 16 && a.NM > 16 ? 24 : 16;
   const int64_t cbytes =
-      a.beta_zero ? 0 : (int64_t)epi_groups(nw) * (MP == 32 ? c_depth<32>() : c_depth<16>()) * CHUNK_BYTES;
+      a.beta_zero ? 0 : (int64_t)epi_groups(nw) * (MP == 32 ? c_depth<32>() : c_depth<16>()) * CRING;
   static_assert(c_depth<16>() == c_depth<64>(), "ring depth");
-  // the deepest A' ring that fits beside B' and the old-C rings (one stage at MP = 64)
+  // the deepest A' ring that fits beside B' and the old-C rings (one stage at MP = 64); at MP = 32 two stages where
+  // rows are read element by element, which a third stage would leave 28 KB of L1 (FP64 32 x 8 out of a block,
+  // 2^18 rows: 69 us with three, 60 with two; FP32 100 and 81)
   a.nast = 0;
-  for (int ns = MAXAST; ns >= 1 && a.nast == 0; ns--)
+  for (int ns = MP == 32 && !a.vec ? 2 : MAXAST; ns >= 1 && a.nast == 0; ns--)
     if (HDR + (int64_t)a.bbytes + (int64_t)ns * a.astage + cbytes <= h->dev.smem_optin) a.nast = ns;
   if (a.nast == 0) {
     set_error("split precision TSMM: tiles do not fit in shared memory");
