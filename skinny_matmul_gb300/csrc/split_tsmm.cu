@@ -195,10 +195,10 @@ __device__ __forceinline__ double alpha_b(const Args& p, int m, int n) {
   return ((n & 1) == 0) ? ((m & 1) == 0 ? ar : -ai) : ((m & 1) == 0 ? ai : ar);
 }
 
-// A row values of this thread's part of the columns (HALF values) for tile row r0 + row, widened
-// to double (exact for float)
-template <int HALF, typename T>
-__device__ __forceinline__ void load_row(const Args& p, int64_t r0, int row, int rows, int m0, double (&v)[HALF]) {
+// A row values of this thread's part of the columns (HALF values) for tile row r0 + row, as they are stored or
+// widened to double (exact for float)
+template <int HALF, typename T, typename V>
+__device__ __forceinline__ void load_row(const Args& p, int64_t r0, int row, int rows, int m0, V (&v)[HALF]) {
   const bool ok = row < rows;
   const T* a = static_cast<const T*>(p.A) + (r0 + row) * p.lda + m0;
   if (ok && p.vec && m0 + HALF <= p.M) {
@@ -221,7 +221,7 @@ __device__ __forceinline__ void load_row(const Args& p, int64_t r0, int row, int
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < HALF; j++) v[j] = (ok && m0 + j < p.M) ? a[j] : 0.0;
+    for (int j = 0; j < HALF; j++) v[j] = (ok && m0 + j < p.M) ? a[j] : T(0);
   }
 }
 
@@ -473,15 +473,21 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
   if (warp < NSL) {
     // ---- slicers: row = tid / 2, columns [m0, m0 + PART) ------------------------------------
     const int row = tid / TPS, part = tid % TPS, m0 = part * PART;
-    double v[PART];
+    // FP32 values are widened when they are used: the conversions wait for the loads, and right behind them
+    // held up the MMAs of the tile before (32 x 8, odd leading dimension, 2^18 rows: 78 us, 60 without; 32 x 32 72 and
+    // 64).  Not at MP = 64, whose 32 conversions a thread then hold up the slicing (64 x 64, 2^14 rows: 33 us and 35).
+    std::conditional_t<MP <= 32, T, double> next[PART];
     auto load_tile = [&](int it) {
       const int64_t r1 = row0 + it * rstep;
-      load_row<PART, T>(p, r1, row, (int)((p.K - r1) < ROWS ? (p.K - r1) : ROWS), m0, v);
+      load_row<PART, T>(p, r1, row, (int)((p.K - r1) < ROWS ? (p.K - r1) : ROWS), m0, next);
     };
     if (nt > 0) load_tile(0);
     int s = 0, es = 0;
     uint32_t sph = 1, eph = 1;  // parities of the releases waited for: the round before
     for (int it = 0; it < nt; it++) {
+      double v[PART];
+#pragma unroll
+      for (int j = 0; j < PART; j++) v[j] = next[j];
       uint32_t emax = 0;
 #pragma unroll
       for (int j = 0; j < PART; j++) emax = max(emax, exp_field(v[j]));
@@ -677,10 +683,12 @@ __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
               const int fc[4] = {f.x, f.y, f.z, f.w};
               double out[4];
               // the conversion runs on the FP64 pipe, next to the beta FMA: on all columns without
-              // beta, on half of them with it (16 x 16 with beta: 527 us with none, 503 with half)
+              // beta, on half of them with it (16 x 16 with beta: 527 us with none, 503 with half); with FP32 storage,
+              // whose values that pipe narrows and widens too, on none at MP = 16 or with beta (2^18 rows, all / none:
+              // 16 x 16 45/41 us, 8 x 32 68/55, 64 x 64 with beta 193/188; but 48 x 48 without 168/174)
 #pragma unroll
               for (int x = 0; x < 4; x++)
-                out[x] = !HASC || x < 2 ? window_cvt(level_window<MP>(raw, x), e + fc[x] - 1086)
+                out[x] = (sizeof(T) == 8 ? !HASC || x < 2 : !HASC && MP > 16) ? window_cvt(level_window<MP>(raw, x), e + fc[x] - 1086)
                                         : window_int(level_window<MP>(raw, x), e + fc[x]);
               if constexpr (HASC) {
                 if (!p.cplx || p.beta[1] == 0.0) {  // a real beta scales both parts of a complex C alike
