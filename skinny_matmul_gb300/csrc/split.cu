@@ -699,7 +699,9 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   //     2^22: 8x8 17.2/15.3, 16x16 20.5/16.5, 32x8 21.8/19.1, 32x32 27.7/28.4; at 2^21 12.4/13.4, 15.9/16.4,
   //     16.5/18.1 and (24x24) 24.2/22.4.  4x16 at 2^22 17.9/18.8, 4x32 at 2^23 27.1/28.3.
   //   * the wide kernel's blocks of 64 x 64 filled by a quarter of a 32 x 32 or 4 x 64 at least (128
-  //     cells where the stages fold, else 256 a block).
+  //     cells where the stages fold, else 256 a block).  With a width below 8 it does not win over bulk copies of
+  //     the CUDA-core kernel where its own are row by row (2^18 rows, 4x32 72/60, with an odd leading dimension
+  //     72/114; 4x64 141/97 and 141/196; out of a wide block, where neither has any, 4x32 114/115, 6x32 141/117).
   // The autotuner can override per shape.
   const bool wide = M > 16 || N > 16;
   const int64_t sym_w = (A == B && lda == ldb && M == N) ? 1 : 0;
@@ -707,9 +709,11 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   const int64_t nblk_w = sym_w ? bm * (bm + 1) / 2 : bm * bn;
   const int64_t per_blk = (M <= 32 && N <= 32) ? 128 : 256;
   const bool widths_win = M >= 4 && N >= 4 && M * N >= 32;
+  const bool dense_w = lda == M && ldb == N && (uintptr_t)A % 16 == 0 && (uintptr_t)B % 16 == 0;
   const int64_t work_min = (M >= 8 && N >= 8) ? (int64_t)1 << 22 : (int64_t)3 << 22;
   if (autoselect &&
-      (K < 4096 || K * M * N < work_min || !widths_win || (wide && M * N < per_blk * nblk_w))) {
+      (K < 4096 || K * M * N < work_min || !widths_win || (wide && M * N < per_blk * nblk_w) ||
+       (wide && (M < 8 || N < 8) && !dense_w && bulk_rows(M, N, A, lda, B, ldb, sym_w != 0)))) {
     set_error("split precision: not selected automatically for this shape");
     return SKINNY_UNSUPPORTED;
   }
