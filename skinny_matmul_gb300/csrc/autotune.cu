@@ -99,6 +99,9 @@ extern "C" skinny_status skinny_autotune(skinny_handle h, int op, skinny_dtype d
   if (tsmm) {
     for (int b : {0, 1, 2, 4}) cands.push_back(LaunchOpts{b, 0, -1});
   } else {
+    // first the launch that an untuned call gets (the plan's own row tile and CTAs per SM, up to 3 of them, or the
+    // row-streaming kernel with all that fit), so that an entry is not slower than none
+    cands.push_back(LaunchOpts{0, 0, -1});
     for (int b : {1, 2})
       for (int r : {0, 64, 128, 256, 512}) cands.push_back(LaunchOpts{b, r, -1});
   }
