@@ -203,7 +203,9 @@ __global__ void __launch_bounds__(TSMTTSM_THREADS, tsmttsm_ctas<Acc>(TM * TN)) t
   int s = 0, sp = 0;              // stage of tile i and of tile i - 1
   uint32_t phase = 0, phase_p = 0;  // and how often (mod 2) the ring has gone round
   const int stages = p.stages;
-  constexpr int UNROLL = TE <= 16 && sizeof(T) == 4 ? 4 : 2;
+  // rows at a time; one for tiles of more than 256 bytes, whose few passes a tile (16 rows, 5 slices) end in half a
+  // step otherwise (complex FP64 40 x 40, 2^16 rows: 915 us with two, 810; double-double 1940 and 1768)
+  constexpr int UNROLL = TE <= 16 && sizeof(T) == 4 ? 4 : TE * (int)sizeof(Acc) > 256 ? 1 : 2;
   for (int i = 0; i < nt; i++) {
     const int64_t r0 = (t_begin + i) * p.rows;
     const int rows = (int)((p.K - r0) < p.rows ? (p.K - r0) : p.rows);
