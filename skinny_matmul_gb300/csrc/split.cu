@@ -166,10 +166,9 @@ __device__ __forceinline__ uint32_t exp_field(double x) {
   return nz ? (ef ? ef : 1u) : 0u;
 }
 
-__device__ __forceinline__ double pow2i(int e) {  // 2^e for e in [-1022, 1023], clamped outside; NONFINITE: NaN
-  if (e > NONFINITE / 2) return __hiloint2double(0x7FF80000, 0);
-  e = e < -1022 ? -1022 : (e > 1023 ? 1023 : e);
-  return __hiloint2double((e + 1023) << 20, 0);
+__device__ __forceinline__ double pow2i(int e) {  // 2^e from -1022 to 1023, 2^-1022 below, NaN above (only NONFINITE gets there)
+  e = min(max(e, -1022), 1024);
+  return __hiloint2double((e + 1023) << 20, e > 1023);
 }
 
 // Slice one unit: 8 consecutive rows of column c into the octet `buf` of a digit buffer

@@ -212,10 +212,9 @@ __device__ __forceinline__ uint32_t exp_field(double x) {
   return e == 0 && (mh | (uint32_t)__double2loint(x)) ? 1u : e;
 }
 
-__device__ __forceinline__ double pow2i(int e) {  // 2^e, clamped to the normal range; NONFINITE: NaN
-  if (e > NONFINITE / 2) return __hiloint2double(0x7FF80000, 0);
-  e = e < -1022 ? -1022 : (e > 1023 ? 1023 : e);
-  return __hiloint2double((e + 1023) << 20, 0);
+__device__ __forceinline__ double pow2i(int e) {  // 2^e from -1022 to 1023, 2^-1022 below, NaN above (only NONFINITE gets there)
+  e = min(max(e, -1022), 1024);
+  return __hiloint2double((e + 1023) << 20, e > 1023);
 }
 
 // GR: how Gram blocks occur (0: none, A and B differ; 1: the only block; 2: among others), so that the
