@@ -405,6 +405,17 @@ skinny_status tsmttsm_rows_run(const DeviceInfo& dev, Workspace& ws, cudaStream_
   return SKINNY_UNSUPPORTED;
 }
 
+// Workspace asked for up to 64 x 64, whatever the tile and the rows: what the cells, padded by at most 7 columns
+// either way, take with all CTAs that any tile may have per SM.  It only grows with M and N, so that a smaller product
+// captured after a larger one on its stream allocates nothing (complex FP64 43 x 45 takes 1.7 times the entries of
+// 48 x 48, whose tiles fit).
+template <typename Acc>
+size_t tsmttsm_workspace(const DeviceInfo& dev, int64_t M, int64_t N) {
+  if (M > 64 || N > 64) return 0;
+  const int64_t ctas = (int64_t)std::max(dev.sms, 1) * tsmttsm_ctas<Acc>(1) + FINISH_MAX_GROUPS;
+  return (size_t)(ctas * round_up(M, 8) * round_up(N, 8)) * sizeof(Acc);
+}
+
 template <typename T, typename Acc>
 skinny_status tsmttsm_run(const DeviceInfo& dev, Workspace& ws, int* err, cudaStream_t st,
                           int64_t M, int64_t N, int64_t K, const T* A, int64_t lda, T alpha,
@@ -416,7 +427,7 @@ skinny_status tsmttsm_run(const DeviceInfo& dev, Workspace& ws, int* err, cudaSt
   TsmttsmPlan pl;
   skinny_status s = tsmttsm_plan<T, Acc>(dev, M, N, K, A, lda, B, ldb, gram, o, pl);
   if (s != SKINNY_OK) return s;
-  s = workspace_ensure(ws, pl.partials<Acc>(pl.grid), st);
+  s = workspace_ensure(ws, std::max(pl.partials<Acc>(pl.grid), tsmttsm_workspace<Acc>(dev, M, N)), st);
   if (s != SKINNY_OK) return s;
   TsmttsmArgs<T> a;
   a.A = A;

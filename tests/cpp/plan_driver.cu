@@ -53,6 +53,9 @@ static void one(const char* name, int64_t M, int64_t N, int64_t K, int64_t lda, 
     many++;
   }
   ok = ok && (size_t)(entries * a) <= pl.template partials<Acc>(pl.grid);
+  // up to 64 x 64 the workspace asked for covers every plan of the width (one group of cells), and so of smaller ones
+  if (M <= 64 && N <= 64 && groups == 1 && o.blocks_per_sm == 0)
+    ok = ok && pl.template partials<Acc>(pl.grid) <= tsmttsm_workspace<Acc>(dev, M, N);
   if (!ok && bad++ < 20)
     std::printf("%s %lld x %lld K=%lld lda=%lld gram=%d blocks=%d rows=%d: tile %d x %d, %d groups, %d bytes\n", name,
                 (long long)M, (long long)N, (long long)K, (long long)lda, gram, o.blocks_per_sm, o.rows_per_tile, pl.tm,
