@@ -82,6 +82,8 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
 skinny_status split_wide(skinny_handle h, int64_t M, int64_t N, int64_t K, const double* A, int64_t lda,
                          const void* alpha, const double* B, int64_t ldb, const void* beta, double* C,
                          int64_t ldc, cudaStream_t st);
+// Allocates the workspace that split_wide takes with any number of rows, outside of a capture and from 4096 rows on.
+bool split_wide_reserve(skinny_handle h, int64_t M, int64_t N, int64_t K, bool sym, cudaStream_t st);
 // The same with FP32 inputs (in_f32) and / or FP32 output, alpha and beta (out_f32).
 skinny_status split_wide_t(skinny_handle h, bool in_f32, bool out_f32, int64_t M, int64_t N, int64_t K,
                            const void* A, int64_t lda, const void* alpha, const void* B, int64_t ldb,

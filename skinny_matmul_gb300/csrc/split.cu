@@ -710,9 +710,10 @@ skinny_status split_tsmttsm_t(skinny_handle h, bool in_f32, bool out_f32, int64_
   const bool widths_win = M >= 4 && N >= 4 && M * N >= 32;
   const bool dense_w = lda == M && ldb == N && (uintptr_t)A % 16 == 0 && (uintptr_t)B % 16 == 0;
   const int64_t work_min = (M >= 8 && N >= 8) ? (int64_t)1 << 22 : (int64_t)3 << 22;
-  if (autoselect &&
-      (K < 4096 || K * M * N < work_min || !widths_win || (wide && M * N < per_blk * nblk_w) ||
-       (wide && (M < 8 || N < 8) && !dense_w && bulk_rows(M, N, A, lda, B, ldb, sym_w != 0)))) {
+  const bool shape_wins = widths_win && !(wide && M * N < per_blk * nblk_w) &&
+                          !(wide && (M < 8 || N < 8) && !dense_w && bulk_rows(M, N, A, lda, B, ldb, sym_w != 0));
+  if (autoselect && (K < 4096 || K * M * N < work_min || !shape_wins)) {
+    if (wide && shape_wins) split_wide_reserve(h, M, N, K, sym_w != 0, st);  // for more rows
     set_error("split precision: not selected automatically for this shape");
     return SKINNY_UNSUPPORTED;
   }

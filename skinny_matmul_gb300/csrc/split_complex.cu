@@ -49,22 +49,27 @@ skinny_status split_complex_tsmttsm(skinny_handle h, int64_t M, int64_t N, int64
     set_error("split precision complex TSMTTSM: M, N <= 64");
     return SKINNY_UNSUPPORTED;
   }
+  void*& buf = h->split_ws[st];  // P, at most 128 x 128 doubles, one per stream
+  auto allocate = [&]() {
+    if (!buf) {
+      if (cudaMalloc(&buf, (size_t)4 * CMAX * CMAX * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        buf = nullptr;
+        set_error("split complex: cudaMalloc failed");
+        return false;
+      }
+      h->extra_allocs.push_back(buf);
+    }
+    return true;
+  };
   // auto selection, on top of the real product's: the CUDA-core complex kernel holds out longer against
   // the wide kernel (16x16, us, CUDA-core / split: K = 2^12 19.7/30.9, 2^13 28.6/31.4, 2^14 45.7/33.0)
   if (autoselect && (M > 8 || N > 8) && 4 * K * M * N <= (int64_t)1 << 23) {
+    if (split_wide_reserve(h, 2 * M, 2 * N, K, A == B && lda == ldb && M == N, st)) allocate();  // for more rows
     set_error("split precision: not selected automatically for this shape");
     return SKINNY_UNSUPPORTED;
   }
-  void*& buf = h->split_ws[st];  // P, at most 128 x 128 doubles, one per stream
-  if (!buf) {
-    if (cudaMalloc(&buf, (size_t)4 * CMAX * CMAX * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      buf = nullptr;
-      set_error("split complex: cudaMalloc failed");
-      return SKINNY_NO_MEM;
-    }
-    h->extra_allocs.push_back(buf);
-  }
+  if (!allocate()) return SKINNY_NO_MEM;
   double* P = static_cast<double*>(buf);
   const double one = 1.0, zero = 0.0;
   // same buffer and leading dimension: the real product is a Gram product too

@@ -797,6 +797,30 @@ skinny_status split_wide(skinny_handle h, int64_t M, int64_t N, int64_t K, const
   return split_wide_t(h, false, false, M, N, K, A, lda, alpha, B, ldb, beta, C, ldc, st);
 }
 
+// Row chunks of each of nblk blocks at most, and the workspace they take: two halves of 4096 cells a CTA, then the
+// group sums.  Asked for whatever the rows, so that a capture with more of them finds it.
+static int64_t split_wide_chunks(skinny_handle h, int64_t nblk) {
+  return std::max<int64_t>(1, std::min<int64_t>(h->dev.sms / nblk, (int64_t)15 * splitw::GROUP));
+}
+static size_t split_wide_bytes(skinny_handle h, int64_t nblk) {
+  return (size_t)(split_wide_chunks(h, nblk) * nblk * 2 + nblk * 15) * 4096 * 8;
+}
+
+// A product that AUTO leaves to the CUDA-core kernels for its few rows (4096 at least) allocates what more rows will
+// take here, so that these can be captured into a graph after it on the same stream, as before the rule counted rows.
+// False, and nothing allocated, in a capture or below 4096 rows.
+bool split_wide_reserve(skinny_handle h, int64_t M, int64_t N, int64_t K, bool sym, cudaStream_t st) {
+  using namespace splitw;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (K < 4096 || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const int64_t bm = (M + W - 1) / W, bn = (N + W - 1) / W, nblk = sym ? bm * (bm + 1) / 2 : bm * bn;
+  workspace_ensure(h->ws[st], split_wide_bytes(h, nblk), st);  // (without room: as the larger call finds it)
+  return true;
+}
+
 skinny_status split_wide_t(skinny_handle h, bool in_f32, bool out_f32, int64_t M, int64_t N, int64_t K,
                            const void* A, int64_t lda, const void* alpha, const void* B, int64_t ldb,
                            const void* beta, void* C, int64_t ldc, cudaStream_t st) {
@@ -850,11 +874,10 @@ skinny_status split_wide_t(skinny_handle h, bool in_f32, bool out_f32, int64_t M
   const int smem = (int)(fixed + (int64_t)a.rstages * a.raw_stage);
   const int64_t srows = fold ? 2 * ROWS : ROWS;
   a.nstages = (K + srows - 1) / srows;
-  const int64_t nchunks = std::max<int64_t>(1, std::min<int64_t>({a.nstages, h->dev.sms / a.nblk,
-                                                                   (int64_t)15 * GROUP}));
+  const int64_t nchunks = std::max<int64_t>(1, std::min(a.nstages, split_wide_chunks(h, a.nblk)));
   const int64_t grid = nchunks * a.nblk;
   Workspace& ws = h->ws[st];
-  skinny_status s = workspace_ensure(ws, ((size_t)grid * 2 + (size_t)a.nblk * 15) * 4096 * 8, st);
+  skinny_status s = workspace_ensure(ws, split_wide_bytes(h, a.nblk), st);
   if (s != SKINNY_OK) return s;
   a.partials = (double*)ws.partials;
   a.counter = ws.counter;
