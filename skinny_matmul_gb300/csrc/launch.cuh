@@ -246,13 +246,13 @@ skinny_status tsmttsm_plan(const DeviceInfo& dev, int64_t M, int64_t N, int64_t 
     const int64_t n = std::max<int64_t>((per_cta + rows - 1) / rows, per_cta >= 64 ? 2 : 1);
     const int most_rows = (int)std::min<int64_t>(rows, round_up((per_cta + 1) / (per_cta >= 64 ? 2 : 1), 16));
     rows = (int)std::min<int64_t>(rows, round_up((per_cta + n - 1) / n, 16));
-    // widened types take the largest tiles, so the most row slices: down to three quarters of the rows that
-    // fit, the ones with the fewest passes of the slices over a CTA's tiles, a hand-off counting a quarter
+    // widened types take the largest tiles, so the most row slices: of the rows that fit, the ones with the
+    // fewest passes of the slices over the tiles of the CTA with most, a hand-off counting a quarter
     // (144 rows for 128 slices are two passes, the second nearly empty: complex FP32 7 x 7, 2^20 rows:
     // 749 us, 585 with 128 rows; FP64 and FP32 lose as much as they gain by it, up to 10 %)
     if (widens<T, Acc>()) {
       int64_t fewest = -1;
-      for (int r = most_rows; r >= 16 && 4 * r >= 3 * most_rows; r -= 16) {
+      for (int r = most_rows; r >= 16; r -= 16) {
         const int64_t tiles = ((K + r - 1) / r + ctas - 1) / ctas, passes = tiles * (4 * ((r + RS - 1) / RS) + 1);
         if (fewest < 0 || passes < fewest) {
           fewest = passes;
