@@ -59,14 +59,15 @@ __device__ __forceinline__ void slot_tree(Acc* sm, int n, int E) {
 // written by other CTAs (L2-coherent loads).  Few entries: the threads share the range of partials
 // and a tree joins them (sm: NT entries).  Many: 16 bytes of entries per thread and step, eight
 // partials in flight (a 64 x 64 FP32 sum of 12 partials: 3 us; with four single loads, 12 us).  Few partials of 4096 or
-// more 8-byte entries are better summed one entry a thread, four partials in flight (FP64 128 x 128, 4 partials: 144 us
-// the call, 126; FP32 100 x 100 in FP64, 12 on each level: 284 and 266; but 152 of them 1004 and 1112).
+// more FP64 entries are better summed one entry a thread, four partials in flight (128 x 128, 4 partials: 144 us
+// the call, 126; FP32 100 x 100 in FP64, 12 on each level: 284 and 266; but 152 of them 1004 and 1112; complex FP32 64 x 64
+// with 12 on each level 101 and 129).
 template <typename O, typename Acc, int NT, typename Out>
 __device__ __forceinline__ void sum_partials(const Acc* src, int cnt, int E, Acc* sm, Out out) {
   const int tid = threadIdx.x;
   constexpr int V = sizeof(Acc) < 16 ? 16 / (int)sizeof(Acc) : 1;
   if constexpr (V > 1) {
-    if (E >= NT && E % V == 0 && (V > 2 || E < 4096 || cnt > 32)) {
+    if (E >= NT && E % V == 0 && (!std::is_same<Acc, double>::value || E < 4096 || cnt > 32)) {
       union Pack {
         uint4 w;
         Acc v[V];
