@@ -64,8 +64,18 @@ typedef enum {
   SKINNY_ACC_SPLIT = 2,  /* split precision: values sliced into FP16 digits, products on tcgen05
                             tensor cores with exact FP32 accumulation, recombined in FP64.  R64, C64,
                             and R32 / C32 storage (widened exactly, rounded once to FP32) at the same
-                            widths.  No counterpart in the reference. */
-  SKINNY_ACC_AUTO = 3    /* fastest method meeting the working precision's error bound */
+                            widths.  Elements become fixed-point numbers of 62 bits below the largest of
+                            their column of A or B so far (TSMM: of the row of A, of the column of B), and
+                            digit products below 2^-56 of the largest are dropped: the error is relative to
+                            these largest elements, not to each product.  An element 2^5 or more below
+                            them loses low bits that NATIVE keeps.  An infinity or NaN makes the entries of
+                            C that it enters NaN in TSMTTSM; for TSMM operands must be finite.
+                            No counterpart in the reference. */
+  SKINNY_ACC_AUTO = 3    /* fastest method meeting the working precision's error bound relative to the
+                            largest elements: NATIVE, or for R64 and C64 SPLIT where it is measured faster
+                            (TSMTTSM: real widths, complex doubled, from 4 x 8 on; TSMM: 128 entries of
+                            B or more, complex 16; 4096 rows or more), with what is said there of range
+                            and of infinities and NaN.  Data that need every element's own bits: NATIVE or DD. */
 } skinny_acc;
 
 typedef struct { float x, y; } skinny_c32;  /* same layout as cuFloatComplex  */
@@ -121,7 +131,8 @@ skinny_status skinny_tsmttsm_conj(skinny_handle handle, skinny_dtype dtype, skin
 /* SVQB orthogonalisation of X (K x M row-major, ldx >= M, FP64), in place, entirely on the
  * device; replaces svqb/svqb.cu:72-130 (which runs the eigensolve on the host through MAGMA).
  *   S = X^T X (gram_acc selects the method), d_i = 1/sqrt(S_ii) (0 if S_ii <= 1e-15),
- *   S <- D S D, S = U L U^T (Jacobi, FP64), T = D U diag(1/sqrt(max(1e-15, l))),
+ *   S <- D S D, S = U L U^T (Jacobi: FP64, from M = 8 on FP32 refined and
+ *   finished in FP64), T = D U diag(1/sqrt(max(1e-15, l))),
  *   X <- X T (in-place TSMM).
  * If orth_err_out is non-null, ||Q^T Q - I||_F is computed on the device (double-double Gram)
  * and written there after a stream synchronisation (svqb/svqb.cu:184-211 getL2Error). */

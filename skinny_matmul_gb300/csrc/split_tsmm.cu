@@ -338,7 +338,7 @@ template <int MP, typename T, int NW, bool HASC>
 __global__ void __launch_bounds__(NW * 32, 1) split_tsmm_kernel(const Args p) {
   constexpr int THREADS = NW * 32;
   constexpr int NEP = NW - NSL, EG = epi_groups(NW);
-  constexpr int TPS = NSL * 32 / ROWS;  // slicer threads per row (2 or 4)
+  constexpr int TPS = NSL * 32 / ROWS;  // slicer threads per row (2)
   constexpr int PART = MP / TPS;        // A values per slicer thread
   // old-C chunks in flight per epilogue thread, and the bytes of one (FP32 48 x 48, odd leading dimension, 2^18 rows:
   // 242 us with as many chunks as FP64 in slots of twice their size, 200)

@@ -49,9 +49,9 @@
 //   * Bound: a stage of 16 x (64 + 64) values takes ~1650 clocks.  The MMAs alone take ~1400 (900 of
 //     products; operands from shared memory), slicing alone ~1400 (~25 instructions a value, two
 //     thirds of the issue slots), and a TMA copy of the same rows would take ~700.  With 8 warps that
-//     sliced and drained by turns and voted
-//     on the exponents of each stage it was 3600: each step of a stage (two mbarriers, the vote, the
-//     drain) was waited out by all of them.  Measured, K rows: f64 64 x 64, K = 2^20, 794 -> 389 us;
+//     sliced and drained by turns and voted on the exponents of each stage it was 3600: each step of a
+//     stage (two mbarriers, the vote, the drain) was waited out by all of them.
+//     Measured, K rows: f64 64 x 64, K = 2^20, 794 -> 389 us;
 //     32 x 32, K = 2^22, 1252 -> 686; 48 x 24, K = 2^20, 714 -> 325; Gram 64, K = 2^20, 738 -> 364;
 //     rows of 80 (64 x 64, K = 2^20) 776 -> 583; f32 64 x 64, K = 2^18, 308 -> 146.
 //   * Blocks of 64 x 64 (M or N > 64) run in the same launch, as do the row chunks of every

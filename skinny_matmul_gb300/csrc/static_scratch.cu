@@ -30,7 +30,7 @@ extern template skinny_status tsmttsm_dispatch<double, double>(const TsmttsmPlan
 constexpr size_t kStaticCounterBytes = 256;            // 64 ticket counters, cleared per call
 constexpr size_t kStaticErrOffset = 256;               // device error word (bounded waits)
 constexpr size_t kStaticHeaderBytes = 512;
-constexpr size_t kStaticPartialBytes = (size_t)16 << 20;  // CTA partials: grid * M * N doubles
+constexpr size_t kStaticPartialBytes = (size_t)16 << 20;  // CTA partials (padded cells) and group sums
 // Largest M * N: the CUDA-core kernel reduces through at most 64 groups of 256 cells of 8 x 8
 // entries in FP64 (tsmttsm_plan), i.e. 2^20 entries of C; 2^20 * 8 bytes fills half the array,
 // so at least two CTAs share the rows at the limit.

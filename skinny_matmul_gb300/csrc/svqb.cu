@@ -59,10 +59,9 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
   return y;
 }
 
-// Cyclic Jacobi (n players, n - 1 rounds a sweep, n / 2 rotations a round) on the matrix in buffer A0
-// XX  FP64: V <- V J (columns in slot order); FP32:
-// the rotations of round i go to log[32 i ..] (cosine, sine per pair; log points to
-// this lane's), for eig_replay_kernel.
+// Cyclic Jacobi (n players, n - 1 rounds a sweep, n / 2 rotations a round) on the matrix in A, which changes
+// between two buffers (cur: the one that holds it).  FP64: V <- V J (columns in slot order).  FP32: the rotations
+// of round i go to log[32 i ..] (cosine, sine per pair; log points to this lane's), for eig_replay_kernel.
 //
 // A round is one pass: the pairs (k, l) of pairs cut the matrix into 2 x 2 blocks, each is rotated
 // from both sides by one lane and written, with its mirror image, into the other buffer.  The last
@@ -601,9 +600,10 @@ static skinny_status svqb_scratch(skinny_handle h, cudaStream_t st, double*& out
 // T from the Gram matrix S: eigenvectors to FP32 accuracy, two steps of refinement and two Newton
 // steps towards orthonormality in FP64 (products of M x M matrices, spread over the GPU), then FP64
 // Jacobi sweeps for what is left.  The matrix the sweeps start from, X^T A X, is formed with exact
-// products and sums: rounding it would move the smallest eigenvalues by u times the largest.  M = 64 with a well-conditioned block: 5.4 ms -> 0.28 ms
-// (157 us of it the FP32 Jacobi, 29 the last kernel); condition 1e8, where FP64 sweeps are left: 11.4
-// -> 4.8 ms.  ||Q^T Q - I|| falls with it (M = 64: 4.9e-14 -> 1.5e-14; condition 100: 2e-12 -> 5e-13).
+// products and sums: rounding it would move the smallest eigenvalues by u times the largest.  M = 64 with a
+// well-conditioned block: 5.4 ms -> 0.28 ms (157 us of it the FP32 Jacobi, 29 the last kernel); condition 1e8,
+// where FP64 sweeps are left: 11.4 -> 4.8 ms.  ||Q^T Q - I|| falls with it (M = 64: 4.9e-14 -> 1.5e-14; condition
+// 100: 2e-12 -> 5e-13).
 static skinny_status svqb_transform(const double* S, int M, double* T, double* ws, double* d, int* info,
                                     cudaStream_t st) {
   static SmemAttr attr32, attr64;

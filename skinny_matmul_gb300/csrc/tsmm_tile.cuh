@@ -1,10 +1,11 @@
 // tsmm_tile.cuh -- TSMM on the FP32 pipe (float, complex float): C(KxN) = alpha A(KxM) B(MxN) + beta C,
 // C may be A.
 //
-// Replaces the row-per-thread tsmm_kernel (tsmm.cuh) for these types beyond the narrowest widths.
+// Replaces the row-per-thread tsmm_kernel (tsmm.cuh) for these types but where that is faster (tsmm_walks in
+// launch.cuh: few outputs of rows that share cache lines).
 // There every thread walked a row of A in global memory, one element per load, all lanes of a row
 // loading the same words: L1 wavefronts bounded it at a sixth of HBM rate (20 x 12 out of a block 32
-// wide, 1e6 rows: 107 us; here 27).  Same layouts: A[r*lda+m], B[n*ldb+m], C[r*ldc+n].
+// wide, 1e6 rows: 108 us; here 37).  Same layouts: A[r*lda+m], B[n*ldb+m], C[r*ldc+n].
 //
 // Design:
 //   * Rows stream in tiles through a ring of shared-memory buffers filled by cp.async (16 bytes where

@@ -1,5 +1,5 @@
 // tsmttsm_rows.cuh -- TSMTTSM on CUDA cores for narrow products (padded M x N up to 16 entries, or
-// up to 8 x 8 on the FP32 pipe): C(MxN) = alpha * A^T B + beta * C.
+// up to 8 x 8 for FP32 and complex FP32 storage): C(MxN) = alpha * A^T B + beta * C.
 //
 // Replaces, for these widths, the reference's GENV3X / SPECSMALL blockProductKernel +
 // deviceReduce pairs (tsmttsm/genv3x.cuh:29-81, specsmall.cuh:28-90), which on GB300 stream
